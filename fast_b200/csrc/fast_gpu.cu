@@ -39,6 +39,9 @@ void dfree(T *&p) {
 
 void free_mesh(Ctx &c) {
   c.drop_graphs();
+  c.persist_grid = 0;
+  dfree(c.d_lcol);
+  dfree(c.d_z2);
   for (Bucket &B : c.buckets) {
     dfree(B.d_conn); dfree(B.d_E); dfree(B.d_nu); dfree(B.d_rho); dfree(B.d_slot); dfree(B.d_first);
     dfree(B.d_dN); dfree(B.d_N); dfree(B.d_w);

@@ -225,7 +225,7 @@ struct Ctx {
   double *d_perr = nullptr;
 
   // persistent PCG: systems with at most persist_max_nodes nodes run each
-  // chunk of iterations as one cooperative kernel (grid barriers in d_bar)
+  // chunk of iterations as one cooperative kernel (its exchange words: d_bar)
   int64_t persist_max_nodes = 65536;
   // SpMV lanes per block-row (4, 8, 16 or 32): FP32 takes 4 blocks and FP64 2
   // blocks per lane trip; defaults measured best on a hex20 box (64 blocks per
@@ -265,9 +265,12 @@ struct Ctx {
   bool use_first_touch() const { return first_touch && !zero_fill; }
   int32_t *d_tile_row = nullptr;
   int bulk_ntiles = 0, bulk_vbytes = 0, bulk_cbytes = 0, bulk_grid = 0;
-  int persist_grid = 0;           // blocks of that kernel (0: not yet sized)
-  void *d_bar = nullptr;          // grid barrier words (kBarrierBytes)
-  static constexpr size_t kBarrierBytes = 8192;
+  int persist_grid = 0;           // blocks of that kernel (0: not yet sized) ...
+  int persist_cluster = 0;        // ... and per cluster (1: no cluster)
+  uint16_t *d_lcol = nullptr;     // [nnzb_pad] its list indices of the matrix columns
+  double *d_z2 = nullptr;         // [nnode][4] its second z buffer (either precision)
+  void *d_bar = nullptr;          // exchange words of that kernel (kBarrierBytes)
+  static constexpr size_t kBarrierBytes = 16384;
 
   // CUDA graphs of one chunk of PCG iterations (captured once, replayed)
   cudaGraphExec_t graph_fp64 = nullptr, graph_mixed = nullptr;

@@ -1123,117 +1123,270 @@ cudaError_t launch_build_precond32(Ctx &c, const float *K32, int precond) {
 
 // ---------------------------------------------------------------- persistent PCG
 // For small systems the iteration is latency-bound (five kernels of a few
-// microseconds each).  There one cooperative launch runs a whole chunk of
-// iterations: each block owns a contiguous range of block-rows (nodes), and
-// two grid barriers per iteration separate w = K p (with the p.w partials,
-// the new search direction built on the fly) and the vector updates (with
-// the r.r and z.r partials).  Every block sums the per-block partials itself, in the
-// same fixed order, so the scalars agree in every block without a broadcast
-// and a solve stays bit-reproducible.  Data written by other blocks during
-// the launch (p and the partials) is read through L2 (ld.global.cg).  The
-// scalars and the exit codes are exactly those of pcg_update_fused /
-// pcg_direction_fused; block 0 writes them back to the PcgState at the end.
+// microseconds each).  There one launch runs a whole chunk of iterations: each
+// block owns a contiguous range of block-rows (nodes), and two grid-wide sums
+// per iteration (they are the barriers too) separate w = K p (with the p.w
+// partials, the new search direction built on the fly) and the vector updates
+// (with the r.r and z.r partials).
+//
+// What bounds it: the two sums and the dependent reads between them.  Hence
+//  * sums are fixed-point atomics whose words carry their own arrival counts
+//    (grid_sum): one hop, no partials to read back afterwards, and no fence
+//    where the sum publishes nothing but itself (p.w);
+//  * rows are split by stored blocks, not by count (a degree-3 B-spline row
+//    holds 343 blocks, a hex8 row 27);
+//  * the nodes a block's rows refer to are listed once per launch; their part
+//    of the new direction is built in shared memory once per iteration (one
+//    read of z and p per node instead of one per matrix block: the gathers
+//    through L1 cost more than the matrix), columns become 16-bit list indices;
+//  * the block's matrix rows stay in shared memory for the whole launch as far
+//    as they fit (about 150 KB per SM, 22 MB over the GPU), the rest streams
+//    from L2;
+//  * a thread keeps its node's u, r, z, p and preconditioner in registers;
+//    only z and p go to memory, for the other blocks.
+// Every block forms the same scalars, so all take the same decisions and a
+// solve stays bit-reproducible.  The scalars and the exit codes are exactly
+// those of pcg_update_fused / pcg_direction_fused; block 0 writes them back to
+// the PcgState at the end.  Measured per iteration (rows split evenly, matrix
+// and gathers through L2, release counters and partials read back -> this):
+// hex8 plate tangent, 7,605 nodes, FP32 10.0 -> 6.4 us; hex20, 40,623 nodes,
+// FP32 33.5 -> 19; tied column, 12,526 nodes, FP32 32.6 -> 13; hex20, 4,148
+// nodes, FP64 14.8 -> 7.1; hex8, 525 nodes, FP64 8.8 -> 5.0.
 constexpr int kPersistThreads = 512;
-constexpr uint64_t kBarrierWaitNs = 2000000000ull;  // one barrier wait; then the launch gives up
+constexpr int kPersistSmem = 208 * 1024;   // dynamic shared memory of a block
+constexpr int kPersistRows = 1024;         // resident rows at most (their offsets are kept)
+constexpr int kPersistRowCost = 12;        // a row's vector work in stored blocks (row split)
+constexpr int kHaloNodes = 65536;          // node list: bitmap of this many nodes, 16-bit entries
+constexpr int kHaloBytes = kHaloNodes / 8 + kHaloNodes / 16;  // bitmap, 16-bit rank of each word
+template <typename T> constexpr int kHaloMax = sizeof(T) == 4 ? 4096 : 2560;  // listed nodes per block at most
+constexpr long long kWaitCycles = 4000000000ll;  // about 2 s of SM clock in one wait; then the launch gives up
 
-// Barrier over all blocks of a cooperative launch (grid_barrier below); the
-// words are zeroed before a solve's first launch.
-struct alignas(8) GridBarrier {
-  unsigned int count;  // with gen: one 64-bit arrival counter (8-byte aligned)
-  unsigned int gen;
-  int32_t err;
-  int32_t pad;
+// Words of grid_sum: [2 sets][2 values][3 limbs], zeroed before a launch.
+constexpr int kSumStride = 1;
+struct GridSlots {
+  unsigned long long w[2 * 6 * kSumStride];
 };
-static_assert(sizeof(GridBarrier) <= Ctx::kBarrierBytes, "barrier words exceed their allocation");
+static_assert(sizeof(GridSlots) <= Ctx::kBarrierBytes, "grid_sum words exceed their allocation");
+constexpr int kMaxCluster = 16, kMaxSumBlocks = 148;
 
-__device__ __forceinline__ uint64_t now_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
+// a block's part of grid_sum (shared memory; in a one-cluster grid the other blocks write into it)
+struct SumShared {
+  double red[2][kPersistThreads / 32];
+  double part[2][2][kMaxCluster];  // [phase parity][value][rank]
+  double tot[2][2];
+  int ok[2];
+};
+struct SumState {
+  int phase = 0;
+  unsigned long long seen[2] = {0, 0};  // this lane's word of each set after its last use
+};
+
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank) {
+  uint32_t out;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void cluster_store(double *p, int rank, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_addr(p, rank)), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// One 64-bit arrival counter (the count and gen words read as one), never
-// reset within a solve: thread 0 of each block adds 1 with release semantics
-// and polls with acquire loads until the counter reaches the next multiple of
-// the grid.  (Measured against a sense-reversal barrier whose last arriver
-// resets the count and advances a generation word behind full fences: 11.4
-// against 13.6 us per FP32 PCG iteration on a 22,815-equation tangent; a flag
-// barrier, each block posting its own word and block 0 releasing, was slower
-// still.)  Every wait is bounded: when one runs out the error word is set and
-// every block leaves at its next barrier.
-__device__ bool grid_barrier(GridBarrier *b, int *ok_sh) {
+__device__ __forceinline__ double pow2(int e) {  // 2^e, |e| <= 1022
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
+__device__ __forceinline__ double scale2(double x, int e) {  // x 2^e for |e| <= 2044 in two steps
+  const int h = e / 2;
+  return x * pow2(h) * pow2(e - h);
+}
+
+// Sum over the grid of NV values per thread, the same bits in every block.
+// With ORDERED it is a barrier too: what any thread wrote before it is visible
+// to every thread after it; without, only the sums are exchanged.
+//
+// A value travels as a fixed-point number below 2^E in three limbs of 38, 46
+// and 46 bits, each added to a 64-bit word by an atomic whose top byte counts
+// arrivals: a word whose count has grown by the grid's size is complete, so a
+// block polls the words themselves, and integer addition makes the sum
+// independent of the order of arrival (and exact).  E follows the last value
+// of the same sum (ref) with 40 bits of headroom, which leaves 90 bits below
+// it; a value that does not fit adds a mark instead, and a sum that leaves
+// less than 64 bits is formed again: all blocks see the same words and repeat
+// with the same E.  The words are never reset: a block remembers what it saw.
+// The two sets alternate, so a block cannot add to a word that another block
+// still waits for.  Measured on 148 blocks (cycles): release counter and
+// polls 2,790, then the partials read back 760; these words 1,700 (2,550
+// ORDERED); flags posted by every block and polled by every block 5,000 to
+// 12,000.  Every wait is bounded: when one runs out the block leaves, and the
+// others, whose waits then run out too, follow.
+//
+// A grid of one cluster exchanges its partials through distributed shared
+// memory between two hardware barriers instead.
+template <int NV, bool ORDERED>
+__device__ bool grid_sum(GridSlots *S, SumShared &sh, int CS, int rank, SumState &st, double (&v)[NV],
+                         const double (&ref)[NV]) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr int NW = kPersistThreads / 32;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const double t = warp_sum(v[k]);
+    if (lane == 0) sh.red[k][wid] = t;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile int32_t *verr = &b->err;
-    int ok = *verr == 0;
-    if (ok) {
-      unsigned long long *ctr = reinterpret_cast<unsigned long long *>(&b->count);
-      unsigned long long old, cur;
-      asm volatile("atom.add.release.gpu.u64 %0, [%1], 1;" : "=l"(old) : "l"(ctr) : "memory");
-      const unsigned long long target = (old / gridDim.x + 1) * gridDim.x;
-      asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(cur) : "l"(ctr) : "memory");
-      if (cur < target) {
-        const uint64_t t0 = now_ns();
-        do {
-          if (*verr != 0) { ok = 0; break; }
-          if (now_ns() - t0 > kBarrierWaitNs) { atomicExch(&b->err, 1); ok = 0; break; }
-          asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(cur) : "l"(ctr) : "memory");
-        } while (cur < target);
+  if (CS == (int)gridDim.x) {
+    const int par = st.phase & 1;
+    st.phase++;
+    if (wid == 0) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const double t = warp_sum(lane < NW ? sh.red[k][lane] : 0.0);
+        if (lane < CS) cluster_store(&sh.part[par][k][rank], lane, t);
       }
     }
-    *ok_sh = ok;
+    __syncwarp();
+    cluster_barrier();
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      double t[kMaxCluster];
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; c++) t[c] = c < CS ? sh.part[par][k][c] : 0.0;
+#pragma unroll
+      for (int h = kMaxCluster / 2; h > 0; h /= 2)
+#pragma unroll
+        for (int c = 0; c < h; c++) t[c] += t[c + h];
+      v[k] = t[0];
+    }
+    return true;
+  }
+  if (wid == 0) {
+    double t[NV], res[NV];
+    int E[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      t[k] = warp_sum(lane < NW ? sh.red[k][lane] : 0.0);
+      const double r = fabs(ref[k]);
+      E[k] = r > 0.0 && r < 1e300 ? (int)((__double_as_longlong(r) >> 52) & 2047) - 1023 + 40 : 40;
+      E[k] = max(-860, min(980, E[k]));
+      res[k] = 0.0;
+    }
+    const bool mine = lane < 3 * NV;
+    const int k0 = mine ? lane / 3 : 0, limb = lane - 3 * (lane / 3);
+    if (ORDERED) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    bool ok = true, again = true;
+    while (again) {
+      const int par = st.phase & 1;
+      st.phase++;
+      const double x = (NV > 1 && k0) ? t[NV - 1] : t[0];
+      const int e = (NV > 1 && k0) ? E[NV - 1] : E[0];
+      unsigned long long *w = &S->w[(par * 6 + (mine ? lane : 0)) * kSumStride];
+      // this lane's limb: the mantissa of x shifted to the limb's lowest bit
+      // (bits below 2^(e - 130) are dropped), with the sign of x
+      const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
+      const int xe = (int)((xb >> 52) & 2047);
+      const int sft = xe - 1075 - (e - 38 - 46 * limb);
+      unsigned long long m = xe ? (xb & ((1ull << 52) - 1)) | (1ull << 52) : 0ull;
+      m = sft >= 0 ? (sft < 46 ? m << sft : 0ull) : (sft > -53 ? m >> -sft : 0ull);
+      if (limb > 0) m &= (1ull << 46) - 1;
+      long long add = (long long)xb < 0 ? -(long long)m : (long long)m;
+      if (xe - 1023 >= e) add = limb == 0 ? 1ll << 47 : 0;  // does not fit (or is not finite)
+      unsigned long long cur = 0;
+      const unsigned long long seen = par ? st.seen[1] : st.seen[0];
+      if (mine)
+        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"((1ull << 56) + (unsigned long long)add)
+                     : "memory");
+      // (the lanes poll together: a loop left lane by lane re-reads a word at a time)
+      const long long t0 = clock64();
+      while (true) {
+        if (ORDERED) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(cur) : "l"(w) : "memory");
+        else asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(cur) : "l"(w) : "memory");
+        const bool here = !mine || (unsigned)((cur - seen + (1ull << 55)) >> 56) == gridDim.x;
+        if (__all_sync(0xffffffffu, here)) break;
+        ok = clock64() - t0 <= kWaitCycles;
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      }
+      const long long sum = (long long)(cur - seen - ((unsigned long long)gridDim.x << 56));
+      if (mine) {
+        if (par) st.seen[1] = cur; else st.seen[0] = cur;
+      }
+      again = false;
+      const double d = scale2((double)sum, e - 38 - 46 * (limb < 3 ? limb : 0));
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const bool over = __shfl_sync(0xffffffffu, (int)(sum >= (1ll << 46)), 3 * k) != 0;
+        const double d1 = __shfl_sync(0xffffffffu, d, 3 * k + 1), d2 = __shfl_sync(0xffffffffu, d, 3 * k + 2);
+        res[k] = __shfl_sync(0xffffffffu, d, 3 * k) + (d1 + d2);
+        const int re = (int)((__double_as_longlong(res[k]) >> 52) & 2047) - 1023;
+        if (over) {                                        // a partial did not fit
+          if (E[k] < 980) { E[k] = min(980, E[k] + 80); again = true; }
+          else res[k] = __longlong_as_double(0x7FF8000000000000ll);
+        } else if (re < E[k] - 66 && E[k] > -860) {        // fewer than 64 bits left
+          E[k] = max(-860, res[k] != 0.0 ? re + 20 : E[k] - 60);
+          again = true;
+        }
+      }
+      again = again && ok;
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) sh.tot[0][k] = res[k];
+      sh.ok[0] = ok;
+    }
   }
   __syncthreads();
-  return *ok_sh != 0;
+#pragma unroll
+  for (int k = 0; k < NV; k++) v[k] = sh.tot[0][k];
+  return sh.ok[0] != 0;
 }
 
-template <typename T> struct V4cg;
-template <> struct V4cg<float> {
-  static __device__ __forceinline__ void load(const float *p, float &a, float &b, float &c) {
-    const float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
-    a = v.x; b = v.y; c = v.z;
-  }
-};
-template <> struct V4cg<double> {
-  static __device__ __forceinline__ void load(const double *p, double &a, double &b, double &c) {
-    const double2 v0 = __ldcg(reinterpret_cast<const double2 *>(p));
-    a = v0.x; b = v0.y; c = __ldcg(p + 2);
-  }
-};
-
 // gather of the search direction: x_j = p_j (first iteration of a launch) or
-// x_j = z_j + beta p_j (the direction of this iteration, built from the last
-// one), read through L2
+// x_j = z_j + beta p_j (the direction of this iteration, built from the last one)
 template <typename T>
 struct DirGather {
   const T *p, *z;
   T beta;
   bool plain;
   __device__ __forceinline__ void load(int64_t j, T &a, T &b, T &c) const {
-    V4cg<T>::load(p + 4 * j, a, b, c);
+    V4<T>::load(p + 4 * j, a, b, c);
     if (!plain) {
       T z0, z1, z2;
-      V4cg<T>::load(z + 4 * j, z0, z1, z2);
+      V4<T>::load(z + 4 * j, z0, z1, z2);
       a = z0 + beta * a;
       b = z1 + beta * b;
       c = z2 + beta * c;
     }
   }
 };
+// ... from the block's list in shared memory
+template <typename T>
+struct HaloGather {
+  const T *x;
+  __device__ __forceinline__ void load(int64_t j, T &a, T &b, T &c) const { V4<T>::load(x + 4 * j, a, b, c); }
+};
 
-__device__ __forceinline__ void persist_row_dir(const int32_t *__restrict__ scol, const float *__restrict__ vr,
-                                                int32_t s0, int32_t nbp, int q, const DirGather<float> &x, float &a0,
-                                                float &a1, float &a2) {
-  for (int j = 4 * q; j < nbp; j += 64) {
-    const int4 c = *reinterpret_cast<const int4 *>(scol + s0 + j);
+// one block-row's product, LPR lanes; col / vr at the row's first block
+// (columns as nodes, int32, or as list indices, uint16)
+template <int LPR, typename C, typename X>
+__device__ __forceinline__ void persist_row(const C *col, const float *vr, int32_t nbp, int q, const X &x, float &a0,
+                                            float &a1, float &a2) {
+  for (int j = 4 * q; j < nbp; j += 4 * LPR) {
+    int32_t c[4];
+    if (sizeof(C) == 2) {
+      const ushort4 t = *reinterpret_cast<const ushort4 *>(col + j);
+      c[0] = t.x; c[1] = t.y; c[2] = t.z; c[3] = t.w;
+    } else {
+      const int4 t = *reinterpret_cast<const int4 *>(col + j);
+      c[0] = t.x; c[1] = t.y; c[2] = t.z; c[3] = t.w;
+    }
     float4 v[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) v[k] = *reinterpret_cast<const float4 *>(vr + k * nbp + j);
     float xa0, xa1, xa2, xb0, xb1, xb2, xc0, xc1, xc2, xd0, xd1, xd2;
-    x.load(c.x, xa0, xa1, xa2);
-    x.load(c.y, xb0, xb1, xb2);
-    x.load(c.z, xc0, xc1, xc2);
-    x.load(c.w, xd0, xd1, xd2);
+    x.load(c[0], xa0, xa1, xa2);
+    x.load(c[1], xb0, xb1, xb2);
+    x.load(c[2], xc0, xc1, xc2);
+    x.load(c[3], xd0, xd1, xd2);
     a0 += v[0].x * xa0 + v[1].x * xa1 + v[2].x * xa2 + v[0].y * xb0 + v[1].y * xb1 + v[2].y * xb2 +
           v[0].z * xc0 + v[1].z * xc1 + v[2].z * xc2 + v[0].w * xd0 + v[1].w * xd1 + v[2].w * xd2;
     a1 += v[3].x * xa0 + v[4].x * xa1 + v[5].x * xa2 + v[3].y * xb0 + v[4].y * xb1 + v[5].y * xb2 +
@@ -1242,142 +1395,316 @@ __device__ __forceinline__ void persist_row_dir(const int32_t *__restrict__ scol
           v[6].z * xc0 + v[7].z * xc1 + v[8].z * xc2 + v[6].w * xd0 + v[7].w * xd1 + v[8].w * xd2;
   }
 }
-__device__ __forceinline__ void persist_row_dir(const int32_t *__restrict__ scol, const double *__restrict__ vr,
-                                                int32_t s0, int32_t nbp, int q, const DirGather<double> &x,
-                                                double &a0, double &a1, double &a2) {
-  for (int j = 2 * q; j < nbp; j += 32) {
-    const int2 c = *reinterpret_cast<const int2 *>(scol + s0 + j);
+template <int LPR, typename C, typename X>
+__device__ __forceinline__ void persist_row(const C *col, const double *vr, int32_t nbp, int q, const X &x,
+                                            double &a0, double &a1, double &a2) {
+  for (int j = 2 * q; j < nbp; j += 2 * LPR) {
+    int32_t c[2];
+    if (sizeof(C) == 2) {
+      const ushort2 t = *reinterpret_cast<const ushort2 *>(col + j);
+      c[0] = t.x; c[1] = t.y;
+    } else {
+      const int2 t = *reinterpret_cast<const int2 *>(col + j);
+      c[0] = t.x; c[1] = t.y;
+    }
     double2 v[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) v[k] = *reinterpret_cast<const double2 *>(vr + k * nbp + j);
     double xa0, xa1, xa2, xb0, xb1, xb2;
-    x.load(c.x, xa0, xa1, xa2);
-    x.load(c.y, xb0, xb1, xb2);
+    x.load(c[0], xa0, xa1, xa2);
+    x.load(c[1], xb0, xb1, xb2);
     a0 += v[0].x * xa0 + v[1].x * xa1 + v[2].x * xa2 + v[0].y * xb0 + v[1].y * xb1 + v[2].y * xb2;
     a1 += v[3].x * xa0 + v[4].x * xa1 + v[5].x * xa2 + v[3].y * xb0 + v[4].y * xb1 + v[5].y * xb2;
     a2 += v[6].x * xa0 + v[7].x * xa1 + v[8].x * xa2 + v[6].y * xb0 + v[7].y * xb1 + v[8].y * xb2;
   }
 }
 
-// sum of the G per-block partials at part[0..G), the same in every block
-__device__ __forceinline__ double persist_sum(const double *part, int G, double *sbuf, double *bc) {
-  const double v = threadIdx.x < G ? __ldcg(part + threadIdx.x) : 0.0;
-  const double t = block_sum<kPersistThreads>(v, sbuf);
-  if (threadIdx.x == 0) *bc = t;
-  __syncthreads();
-  const double r = *bc;
-  __syncthreads();
-  return r;
+// largest row in [lo, hi] with srow[row] - base + cost * (row - row0) <= target
+// (the expression does not decrease with the row and is <= target at lo); the
+// whole block narrows the range kPersistThreads-fold per round
+__device__ __forceinline__ int32_t find_row(const int32_t *srow, int32_t lo, int32_t hi, int64_t base, int64_t cost,
+                                            int32_t row0, int64_t target) {
+  while (hi > lo) {
+    const int32_t step = (hi - lo + kPersistThreads - 1) / kPersistThreads;
+    const int64_t row = lo + (int64_t)step * (threadIdx.x + 1);
+    const bool in = row <= hi && (int64_t)srow[row] - base + cost * (row - row0) <= target;
+    lo += step * __syncthreads_count(in);
+    hi = min(hi, lo + step - 1);
+  }
+  return lo;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kPersistThreads, 1)
-pcg_persistent(int64_t nnode, const int32_t *__restrict__ srow, const int32_t *__restrict__ scol,
-               const T *__restrict__ val, T *u, T *r, T *z, T *p, T *p2, T *w, const T *__restrict__ dinv,
-               PcgState *st, double *part_pw, double *part_rr, double *part_zr, GridBarrier *bar, int iters) {
-  __shared__ double sbuf[32];
-  __shared__ double bc;
-  __shared__ int ok_sh;
+struct PersistArgs {
+  int32_t nnode;
+  const int32_t *srow, *scol;
+  uint16_t *lcol;           // [nnzb_pad] scratch: list indices of the rows that stream
+  const T *val;
+  T *u, *r, *z, *z2, *p, *p2, *w;
+  const T *dinv;
+  PcgState *st;
+  GridSlots *slots;
+  int iters;
+};
+
+template <typename T, int LPR>
+__global__ void __launch_bounds__(kPersistThreads, 1) pcg_persistent(PersistArgs<T> A) {
+  extern __shared__ __align__(16) unsigned char psm[];
+  __shared__ SumShared sums;
+  __shared__ T sW[3][kPersistThreads];
+  __shared__ int32_t sRow[kPersistRows + 1];
+  __shared__ int32_t sScan[kPersistThreads / 32 + 1];
+  PcgState *st = A.st;
   if (st->done) return;  // the same value in every block: no block waits alone
-  const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, q = lane & 15;
-  double dot0 = st->dot0, alpha = st->alpha, beta = st->beta, rr = st->rr, err = st->err, pw = st->pw;
+  const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, q = lane % LPR;
+  const int32_t *__restrict__ srow = A.srow, *__restrict__ scol = A.scol;
+  const T *__restrict__ val = A.val, *__restrict__ dinv = A.dinv;
+  const int32_t nnode = A.nnode;
+  int CS, rank;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(CS));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  double dot0 = st->dot0, alpha = st->alpha, beta = st->beta, rr = st->rr, pw = st->pw;
   int iter = st->iter, done = 0;
-  const double tol = st->tol, lenf = st->lenf;
+  const double lenf = st->lenf, stop = st->tol * lenf;
   const int maxit = st->maxit;
-  const int64_t rb = (nnode + G - 1) / G;
-  const int64_t r0 = min(nnode, (int64_t)b * rb), r1 = min(nnode, r0 + rb);
+  // the block's rows [r0, r1): an even share of stored blocks + kPersistRowCost per row
+  const int64_t total = (int64_t)srow[nnode] + (int64_t)kPersistRowCost * nnode;
+  const int32_t r0 = b == 0 ? 0 : find_row(srow, 0, nnode, 0, kPersistRowCost, 0, total * b / G);
+  const int32_t r1 = b == G - 1 ? nnode : find_row(srow, 0, nnode, 0, kPersistRowCost, 0, total * (b + 1) / G);
+  const int64_t s00 = srow[r0];
+  const int32_t nall = (int32_t)(srow[r1] - s00);
+  // the nodes these rows refer to: a bitmap, the rank of each of its words, the list
+  uint32_t *bm = reinterpret_cast<uint32_t *>(psm);
+  uint16_t *wrank = reinterpret_cast<uint16_t *>(psm + kHaloNodes / 8);
+  uint16_t *list = wrank + kHaloNodes / 32;
+  bool halo = nnode <= kHaloNodes;
+  int U = 0;
+  if (halo) {
+    constexpr int WPT = kHaloNodes / 32 / kPersistThreads;  // bitmap words per thread
+    for (int i = 0; i < WPT; i++) bm[tid + i * kPersistThreads] = 0;
+    __syncthreads();
+    for (int i = tid; i < nall; i += kPersistThreads) {
+      const int32_t c = scol[s00 + i];
+      const uint32_t bit = 1u << (c & 31);
+      if (!(bm[c >> 5] & bit)) atomicOr(&bm[c >> 5], bit);
+    }
+    __syncthreads();
+    int cnt = 0;
+    for (int i = 0; i < WPT; i++) cnt += __popc(bm[WPT * tid + i]);
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) sScan[wid] = incl;
+    __syncthreads();
+    int base = 0;
+    for (int i = 0; i < kPersistThreads / 32; i++) {
+      const int t = sScan[i];
+      if (i < wid) base += t;
+      U += t;
+    }
+    halo = U <= kHaloMax<T>;
+    int pos = base + incl - cnt;
+    for (int i = 0; i < WPT; i++) {
+      uint32_t m = bm[WPT * tid + i];
+      wrank[WPT * tid + i] = (uint16_t)pos;
+      while (halo && m) {
+        list[pos++] = (uint16_t)(32 * (WPT * tid + i) + __ffs(m) - 1);
+        m &= m - 1;
+      }
+    }
+    __syncthreads();
+  }
+  auto list_index = [&](int32_t c) {
+    return (uint16_t)(wrank[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u)));
+  };
+  // shared memory: [bitmap, ranks, list, their x] [values, columns of rows [r0, rs)]
+  const int off_x = halo ? (kHaloBytes + 2 * U + 15) / 16 * 16 : 0;
+  const int off_v = halo ? off_x + U * 4 * (int)sizeof(T) : 0;
+  const int blk_bytes = 9 * (int)sizeof(T) + (halo ? 2 : 4);
+  T *xs = reinterpret_cast<T *>(psm + off_x);
+  const int32_t rs = find_row(srow, r0, min(r1, r0 + kPersistRows), s00, 0, r0, (kPersistSmem - off_v) / blk_bytes);
+  const int32_t nblk = (int32_t)(srow[rs] - s00);
+  T *sv = reinterpret_cast<T *>(psm + off_v);
+  unsigned char *scb = psm + off_v + (size_t)9 * sizeof(T) * nblk;
+  uint16_t *sc16 = reinterpret_cast<uint16_t *>(scb);
+  int32_t *sc32 = reinterpret_cast<int32_t *>(scb);
+  {
+    const uint4 *gv = reinterpret_cast<const uint4 *>(val + 9 * s00);
+    uint4 *dv = reinterpret_cast<uint4 *>(sv);
+    for (int i = tid; i < nblk * (9 * (int)sizeof(T) / 4) / 4; i += kPersistThreads) dv[i] = gv[i];
+    if (halo) {
+      for (int i = tid; i < nblk; i += kPersistThreads) sc16[i] = list_index(scol[s00 + i]);
+      for (int i = nblk + tid; i < nall; i += kPersistThreads) A.lcol[s00 + i] = list_index(scol[s00 + i]);
+    } else {
+      for (int i = tid; i < nblk; i += kPersistThreads) sc32[i] = scol[s00 + i];
+    }
+    for (int i = tid; i <= rs - r0; i += kPersistThreads) sRow[i] = (int32_t)(srow[r0 + i] - s00);
+  }
+  // the thread's own node (rows beyond kPersistThreads per block are worked on in memory)
+  const int32_t n = r0 + tid;
+  const bool own = n < r1;
+  T *u = A.u, *r = A.r, *w = A.w;
+  T u0 = 0, u1 = 0, u2 = 0, x0 = 0, x1 = 0, x2 = 0, z0 = 0, z1 = 0, z2 = 0, p0 = 0, p1 = 0, p2_ = 0, D[12];
+#pragma unroll
+  for (int k = 0; k < 12; k++) D[k] = 0;
+  if (own) {
+    V4<T>::load(u + 4 * (int64_t)n, u0, u1, u2);
+    V4<T>::load(r + 4 * (int64_t)n, x0, x1, x2);
+    V4<T>::load(A.p + 4 * (int64_t)n, p0, p1, p2_);
+#pragma unroll
+    for (int k = 0; k < 12; k++)
+      if (k % 4 != 3) D[k] = dinv[12 * (int64_t)n + k];
+  }
+  cluster_barrier();  // (in a one-cluster grid the other blocks' shared memory may now be written)
   // The direction of iteration k+1 is p = z + beta p_k.  Instead of a third
   // barrier before the SpMV, each block builds it on the fly from z and the
-  // last direction (both final after the second barrier) for every gathered
-  // node, and stores it for its own nodes in the other buffer.
-  T *pcur = p, *pnxt = p2;
+  // last direction (both published by the second sum) for every node it needs,
+  // and stores it for its own nodes in the other buffer.  z has two buffers
+  // too: the first sum orders nothing, so a block may write its new z while
+  // another still reads the old one.
+  T *pcur = A.p, *pnxt = A.p2, *z = A.z, *znxt = A.z2;
   bool first = true;
-  int it = 0;
-  for (; it < iters; it++) {
-    const DirGather<T> dir{pcur, z, (T)beta, first};
+  SumState ss;
+  for (int it = 0; it < A.iters; it++) {
+    const T be = (T)beta;
+    const DirGather<T> dir{pcur, z, be, first};
     T *pdir = first ? pcur : pnxt;
-    // w = K p on the block's rows, partial p.w, own rows of p stored
-    double pacc = 0.0;
-    for (int64_t row0 = r0 + 2 * (tid >> 5); row0 < r1; row0 += 2 * (kPersistThreads / 32)) {
-      const int64_t row = row0 + (lane >> 4);
-      const bool live = row < r1;
-      int32_t s0 = 0, nbp = 0;
-      if (live) {
-        s0 = srow[row];
-        nbp = srow[row + 1] - s0;
+    if (halo)
+      for (int i = tid; i < U; i += kPersistThreads) {
+        T a, bb, c;
+        dir.load(list[i], a, bb, c);
+        V4<T>::store(xs + 4 * i, a, bb, c);
       }
+    if (!first) {
+      if (own) {
+        p0 = z0 + be * p0; p1 = z1 + be * p1; p2_ = z2 + be * p2_;
+        V4<T>::store(pdir + 4 * (int64_t)n, p0, p1, p2_);
+      }
+      for (int32_t m = n + kPersistThreads; m < r1; m += kPersistThreads) {
+        T a, bb, c;
+        dir.load(m, a, bb, c);
+        V4<T>::store(pdir + 4 * (int64_t)m, a, bb, c);
+      }
+    }
+    __syncthreads();
+    // w = K p on the block's rows
+    constexpr int RPW = 32 / LPR, STEP = RPW * (kPersistThreads / 32);
+    for (int32_t row0 = r0 + RPW * wid; row0 < r1; row0 += STEP) {
+      const int32_t row = row0 + lane / LPR;
       T a0 = 0, a1 = 0, a2 = 0;
-      persist_row_dir(scol, val + 9 * (int64_t)s0, s0, nbp, q, dir, a0, a1, a2);
+      if (halo) {
+        const HaloGather<T> hx{xs};
+        if (row < rs) {
+          const int32_t s0 = sRow[row - r0], nbp = sRow[row - r0 + 1] - s0;
+          persist_row<LPR>(sc16 + s0, sv + 9 * s0, nbp, q, hx, a0, a1, a2);
+        } else if (row < r1) {
+          const int32_t s0 = srow[row], nbp = srow[row + 1] - s0;
+          persist_row<LPR>(A.lcol + s0, val + 9 * (int64_t)s0, nbp, q, hx, a0, a1, a2);
+        }
+      } else if (row < rs) {
+        const int32_t s0 = sRow[row - r0], nbp = sRow[row - r0 + 1] - s0;
+        persist_row<LPR>(sc32 + s0, sv + 9 * s0, nbp, q, dir, a0, a1, a2);
+      } else if (row < r1) {
+        const int32_t s0 = srow[row], nbp = srow[row + 1] - s0;
+        persist_row<LPR>(scol + s0, val + 9 * (int64_t)s0, nbp, q, dir, a0, a1, a2);
+      }
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
+      for (int o = LPR / 2; o > 0; o >>= 1) {
         a0 += __shfl_xor_sync(0xffffffffu, a0, o);
         a1 += __shfl_xor_sync(0xffffffffu, a1, o);
         a2 += __shfl_xor_sync(0xffffffffu, a2, o);
       }
-      if (live && q == 0) {
-        V4<T>::store(w + 4 * row, a0, a1, a2);
-        T x0, x1, x2;
-        dir.load(row, x0, x1, x2);
-        if (!first) V4<T>::store(pdir + 4 * row, x0, x1, x2);
-        pacc += (double)x0 * a0 + (double)x1 * a1 + (double)x2 * a2;
+      if (row < r1 && q == 0) {
+        const int32_t l = row - r0;
+        if (l < kPersistThreads) {
+          sW[0][l] = a0; sW[1][l] = a1; sW[2][l] = a2;
+        } else {
+          V4<T>::store(w + 4 * (int64_t)row, a0, a1, a2);
+        }
       }
     }
     pcur = pdir;
-    pnxt = (pdir == p) ? p2 : p;
+    pnxt = (pdir == A.p) ? A.p2 : A.p;
     first = false;
-    double t = block_sum<kPersistThreads>(pacc, sbuf);
-    if (tid == 0) part_pw[b] = t;
-    if (!grid_barrier(bar, &ok_sh)) { done = kDoneBarrierTimeout; break; }
-    pw = persist_sum(part_pw, G, sbuf, &bc);
+    __syncthreads();
+    // p.w
+    double s1[1] = {0.0};
+    T w0 = 0, w1 = 0, w2 = 0;
+    if (own) {
+      w0 = sW[0][tid]; w1 = sW[1][tid]; w2 = sW[2][tid];
+      s1[0] = (double)p0 * w0 + (double)p1 * w1 + (double)p2_ * w2;
+    }
+    for (int32_t m = n + kPersistThreads; m < r1; m += kPersistThreads) {
+      T a, bb, c, e0, e1, e2;
+      V4<T>::load(pcur + 4 * (int64_t)m, a, bb, c);
+      V4<T>::load(w + 4 * (int64_t)m, e0, e1, e2);
+      s1[0] += (double)a * e0 + (double)bb * e1 + (double)c * e2;
+    }
+    const double ref1[1] = {pw != 0.0 ? pw : dot0};
+    if (!grid_sum<1, false>(A.slots, sums, CS, rank, ss, s1, ref1)) { done = kDoneBarrierTimeout; break; }
+    pw = s1[0];
     alpha = dot0 / pw;
     if (!(alpha > 0.0) || !isfinite(pw) || !isfinite(alpha)) { done = 3; break; }
-    // u += alpha p; r -= alpha w; z = Dinv r; partials r.r, z.r
+    // u += alpha p; r -= alpha w; z = Dinv r; r.r, z.r
     const T al = (T)alpha;
-    double rra = 0.0, zra = 0.0;
-    for (int64_t n = r0 + tid; n < r1; n += kPersistThreads) {
-      T u0, u1, u2, p0, p1, p2_, x0, x1, x2, w0, w1, w2, z0, z1, z2;
-      V4<T>::load(u + 4 * n, u0, u1, u2);
-      V4<T>::load(pcur + 4 * n, p0, p1, p2_);
-      V4<T>::load(r + 4 * n, x0, x1, x2);
-      V4<T>::load(w + 4 * n, w0, w1, w2);
-      u0 = u0 + al * p0; u1 = u1 + al * p1; u2 = u2 + al * p2_;
+    double s2[2] = {0.0, 0.0};
+    if (own) {
       x0 = x0 + (-al) * w0; x1 = x1 + (-al) * w1; x2 = x2 + (-al) * w2;
-      apply_dinv(dinv + 12 * n, x0, x1, x2, z0, z1, z2);
-      V4<T>::store(u + 4 * n, u0, u1, u2);
-      V4<T>::store(r + 4 * n, x0, x1, x2);
-      V4<T>::store(z + 4 * n, z0, z1, z2);
-      rra += (double)x0 * x0 + (double)x1 * x1 + (double)x2 * x2;
-      zra += (double)z0 * x0 + (double)z1 * x1 + (double)z2 * x2;
+      apply_dinv(D, x0, x1, x2, z0, z1, z2);
+      V4<T>::store(znxt + 4 * (int64_t)n, z0, z1, z2);
+      u0 = u0 + al * p0; u1 = u1 + al * p1; u2 = u2 + al * p2_;
+      s2[0] = (double)x0 * x0 + (double)x1 * x1 + (double)x2 * x2;
+      s2[1] = (double)z0 * x0 + (double)z1 * x1 + (double)z2 * x2;
     }
-    t = block_sum<kPersistThreads>(rra, sbuf);
-    if (tid == 0) part_rr[b] = t;
-    t = block_sum<kPersistThreads>(zra, sbuf);
-    if (tid == 0) part_zr[b] = t;
-    if (!grid_barrier(bar, &ok_sh)) { done = kDoneBarrierTimeout; break; }
-    rr = persist_sum(part_rr, G, sbuf, &bc);
-    const double zr = persist_sum(part_zr, G, sbuf, &bc);
+    for (int32_t m = n + kPersistThreads; m < r1; m += kPersistThreads) {
+      T a, bb, c, e0, e1, e2, f0, f1, f2, g0, g1, g2;
+      V4<T>::load(pcur + 4 * (int64_t)m, a, bb, c);
+      V4<T>::load(w + 4 * (int64_t)m, e0, e1, e2);
+      V4<T>::load(u + 4 * (int64_t)m, f0, f1, f2);
+      V4<T>::store(u + 4 * (int64_t)m, f0 + al * a, f1 + al * bb, f2 + al * c);
+      V4<T>::load(r + 4 * (int64_t)m, f0, f1, f2);
+      f0 = f0 + (-al) * e0; f1 = f1 + (-al) * e1; f2 = f2 + (-al) * e2;
+      apply_dinv(dinv + 12 * (int64_t)m, f0, f1, f2, g0, g1, g2);
+      V4<T>::store(r + 4 * (int64_t)m, f0, f1, f2);
+      V4<T>::store(znxt + 4 * (int64_t)m, g0, g1, g2);
+      s2[0] += (double)f0 * f0 + (double)f1 * f1 + (double)f2 * f2;
+      s2[1] += (double)g0 * f0 + (double)g1 * f1 + (double)g2 * f2;
+    }
+    { T *t = z; z = znxt; znxt = t; }
+    const double ref2[2] = {rr, dot0};
+    if (!grid_sum<2, true>(A.slots, sums, CS, rank, ss, s2, ref2)) { done = kDoneBarrierTimeout; break; }
+    rr = s2[0];
+    const double zr = s2[1], next_beta = zr / dot0, rlen = sqrt(rr);
     iter += 1;
-    err = sqrt(rr) / lenf;
-    if (err < tol) { done = 1; break; }
-    if (!isfinite(err)) { done = 3; break; }
+    if (rlen < stop) { done = 1; break; }
+    if (!isfinite(rlen)) { done = 3; break; }
     if (iter >= maxit) { done = 2; break; }
-    beta = zr / dot0;
+    beta = next_beta;
     dot0 = zr;
   }
-  // leave the direction the per-kernel iteration expects in p: the next one
-  // (z + beta p) when the chunk ran out, else the last one used
+  // leave u, r and, in p, the direction the per-kernel iteration expects: the
+  // next one (z + beta p) when the chunk ran out, else the last one used
   if (done != kDoneBarrierTimeout) {
     const bool next = (done == 0);
-    if (next || pcur != p) {
-      const T be = (T)beta;
-      for (int64_t n = r0 + tid; n < r1; n += kPersistThreads) {
-        T p0, p1, p2_, z0, z1, z2;
-        V4<T>::load(pcur + 4 * n, p0, p1, p2_);
+    const T be = (T)beta;
+    if (own) {
+      if (next) { p0 = z0 + be * p0; p1 = z1 + be * p1; p2_ = z2 + be * p2_; }
+      V4<T>::store(A.p + 4 * (int64_t)n, p0, p1, p2_);
+      V4<T>::store(u + 4 * (int64_t)n, u0, u1, u2);
+      V4<T>::store(r + 4 * (int64_t)n, x0, x1, x2);
+    }
+    if (next || pcur != A.p) {
+      for (int32_t m = n + kPersistThreads; m < r1; m += kPersistThreads) {
+        T a, bb, c, e0, e1, e2;
+        V4<T>::load(pcur + 4 * (int64_t)m, a, bb, c);
         if (next) {
-          V4<T>::load(z + 4 * n, z0, z1, z2);
-          p0 = z0 + be * p0; p1 = z1 + be * p1; p2_ = z2 + be * p2_;
+          V4<T>::load(z + 4 * (int64_t)m, e0, e1, e2);
+          a = e0 + be * a; bb = e1 + be * bb; c = e2 + be * c;
         }
-        V4<T>::store(p + 4 * n, p0, p1, p2_);
+        V4<T>::store(A.p + 4 * (int64_t)m, a, bb, c);
       }
     }
   }
@@ -1386,11 +1713,12 @@ pcg_persistent(int64_t nnode, const int32_t *__restrict__ srow, const int32_t *_
     st->alpha = alpha;
     st->beta = beta;
     st->rr = rr;
-    st->err = err;
+    st->err = sqrt(rr) / lenf;
     st->pw = pw;
     st->iter = iter;
     st->done = done;
   }
+  cluster_barrier();  // no block leaves while another may still write its shared memory
 }
 
 // ---------------------------------------------------------------- batched PCG
@@ -1405,6 +1733,14 @@ pcg_persistent(int64_t nnode, const int32_t *__restrict__ srow, const int32_t *_
 // largest first, so the block scheduler starts the long ones early.
 constexpr int kBatchThreads = 256;
 constexpr int kBatchCluster = 2;  // measured: 2 -> 1.83 s, 4 -> 1.91 s, 8 -> 2.11 s on the 1024-cantilever ensemble
+
+template <typename T> struct V4cg;
+template <> struct V4cg<double> {
+  static __device__ __forceinline__ void load(const double *p, double &a, double &b, double &c) {
+    const double2 v0 = __ldcg(reinterpret_cast<const double2 *>(p));
+    a = v0.x; b = v0.y; c = __ldcg(p + 2);
+  }
+};
 
 template <int CS>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(kBatchThreads, 2)
@@ -1575,54 +1911,91 @@ cudaError_t launch_pcg_batch(Ctx &c, int nprob, const int32_t *d_order, const in
   return cudaGetLastError();
 }
 
-// k iterations of the persistent kernel; false when the system is too large
-// for it (the caller then uses the per-kernel iteration)
-// (reset_barrier false: inside a graph's loop body, where the barrier words
-// were reset before the loop and every completed launch leaves them reset)
+// lanes per block-row of the persistent kernel: a lane takes 4 FP32 or 2 FP64
+// blocks per trip, so rows of up to 32 blocks (hex8: 27) fill 8 FP32 lanes
+// (16 lanes would idle half of each warp), longer ones 16
+static bool persist_short_rows(const Ctx &c) { return c.nnzb_pad <= 36 * c.nnode; }
+
+static auto persist_kernel(const Ctx &c, float) {
+  return persist_short_rows(c) ? pcg_persistent<float, 8> : pcg_persistent<float, 16>;
+}
+static auto persist_kernel(const Ctx &, double) { return pcg_persistent<double, 16>; }
+
+// k iterations of the persistent kernel (use_persistent(c) holds)
 template <typename T>
-static cudaError_t launch_persistent(Ctx &c, const T *val, T *u, T *r, T *z, T *p, T *p2, T *w, const T *dinv,
-                                     int k, bool reset_barrier = true) {
-  cudaError_t e = reset_barrier ? cudaMemsetAsync(c.d_bar, 0, sizeof(GridBarrier), c.stream) : cudaSuccess;
+static cudaError_t launch_persistent(Ctx &c, const T *val, T *u, T *r, T *z, T *p, T *p2, T *w, const T *dinv, int k) {
+  cudaError_t e = cudaMemsetAsync(c.d_bar, 0, sizeof(GridSlots), c.stream);
   if (e != cudaSuccess) return e;
-  int64_t nn = c.nnode;
-  const int32_t *srow = c.d_srow, *scol = c.d_scol;
-  PcgState *st = c.d_state;
-  double *pa = c.d_partials, *pb = c.d_partials + 2048, *pc = c.d_partials + 4096;
-  GridBarrier *bar = static_cast<GridBarrier *>(c.d_bar);
-  // a cooperative launch (all blocks resident), also as a node of a captured graph
+  const PersistArgs<T> a{(int32_t)c.nnode, c.d_srow, c.d_scol, c.d_lcol, val, u, r, z, reinterpret_cast<T *>(c.d_z2),
+                         p, p2, w, dinv, c.d_state, static_cast<GridSlots *>(c.d_bar), k};
+  // all blocks resident: one cluster, or a cooperative launch; also as a node of a captured graph
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(c.persist_grid);
   cfg.blockDim = dim3(kPersistThreads);
+  cfg.dynamicSmemBytes = kPersistSmem;
   cfg.stream = c.stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
+  if (c.persist_cluster > 1) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c.persist_cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, pcg_persistent<T>, nn, srow, scol, val, u, r, z, p, p2, w, dinv, st, pa, pb, pc, bar, k);
+  e = cudaLaunchKernelEx(&cfg, persist_kernel(c, T(0)), a);
   c.launches++;
   return e;
 }
 
-// small enough, and one block of the kernel fits on every SM (sized once)
+// small enough, and the kernel's blocks fit on the device together (sized once per mesh)
 static bool use_persistent(Ctx &c) {
   if (c.nnode <= 0 || c.nnode > c.persist_max_nodes) return false;
   if (c.persist_grid == 0) {
-    int a = 0, b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pcg_persistent<double>, kPersistThreads, 0) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, pcg_persistent<float>, kPersistThreads, 0) != cudaSuccess ||
-        a < 1 || b < 1) {
+    bool fits = true, cluster = true;
+    auto sized = [&](auto kern) {
+      int a = 0, n = 0;
+      fits = fits &&
+             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistSmem) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kern, kPersistThreads, kPersistSmem) == cudaSuccess &&
+             a >= 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(kMaxCluster);
+      cfg.blockDim = dim3(kPersistThreads);
+      cfg.dynamicSmemBytes = kPersistSmem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = kMaxCluster;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      cluster = cluster && fits &&
+                cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
+    };
+    sized(pcg_persistent<double, 16>);
+    sized(pcg_persistent<float, 16>);
+    sized(pcg_persistent<float, 8>);
+    if (!c.d_lcol && fits)
+      fits = cudaMalloc((void **)&c.d_lcol, sizeof(uint16_t) * std::max<int64_t>(4, c.nnzb_pad)) == cudaSuccess &&
+             cudaMalloc((void **)&c.d_z2, sizeof(double) * 4 * c.nnode) == cudaSuccess;
+    if (!fits) {
       cudaGetLastError();
       c.persist_max_nodes = 0;
       return false;
     }
-    c.persist_grid = 1;  // sized per system below (partials: at most 2048 blocks)
-  }
-  {
-    // one block per SM (measured faster than fewer, fuller blocks), not more than one per 32 rows
-    int64_t g = (c.nnode + 31) / 32;
-    if (g > c.sm_count) g = c.sm_count;
-    c.persist_grid = (int)(g < 1 ? 1 : g);
+    cudaGetLastError();
+    // one block per SM (measured faster than fewer, fuller blocks), not more
+    // than one per 32 rows.  Up to twice the largest cluster's blocks the
+    // system goes to one cluster: its sums need no L2 (525 nodes: 5.7 us an
+    // iteration on 16 blocks in a cluster, 6.1 on 17 without); beyond that the
+    // longer row ranges cost more than the sums save.
+    const int64_t g = std::max<int64_t>(1, (c.nnode + 31) / 32);
+    c.persist_grid = (int)std::min<int64_t>(g, std::min(c.sm_count, kMaxSumBlocks));
+    c.persist_cluster = 1;
+    if (cluster && g <= 2 * kMaxCluster) c.persist_cluster = c.persist_grid = (int)std::min<int64_t>(g, kMaxCluster);
   }
   return true;
 }
@@ -1827,9 +2200,8 @@ cudaError_t record_pcg(Ctx &c, bool mixed, bool warm, double tol, const double *
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // small systems iterate in the persistent cooperative kernel (as the
-  // launched solves do), a chunk per loop pass; its barrier words reset once
+  // launched solves do), a chunk per loop pass
   const bool persist = use_persistent(c);
-  if (persist && (e = cudaMemsetAsync(c.d_bar, 0, sizeof(GridBarrier), c.stream)) != cudaSuccess) return e;
   // the WHILE node, appended to the graph being captured on c.stream
   cudaStreamCaptureStatus cs;
   cudaGraph_t g = nullptr;
@@ -1858,11 +2230,11 @@ cudaError_t record_pcg(Ctx &c, bool mixed, bool warm, double tol, const double *
   if (e == cudaSuccess) {
     cudaError_t el = cudaSuccess;
     if (persist && mixed) {
-      el = launch_persistent<float>(c, c.d_Ks32, c.s_x, c.s_r, c.s_z, c.s_p, c.s_p2, c.s_w, c.s_dinv, chunk, false);
+      el = launch_persistent<float>(c, c.d_Ks32, c.s_x, c.s_r, c.s_z, c.s_p, c.s_p2, c.s_w, c.s_dinv, chunk);
       mixed_reliable(c);
     } else if (persist) {
       el = launch_persistent<double>(c, c.d_Ks, c.d_u, c.d_r, c.d_z, c.d_p, c.d_p2, c.d_w, c.d_dinv,
-                                     chunk < 64 ? 64 : chunk, false);
+                                     chunk < 64 ? 64 : chunk);
     } else if (mixed) {
       mixed_chunk(c, chunk);
     } else {
