@@ -681,7 +681,13 @@ __global__ void __launch_bounds__(256) reliable_scalar(PcgState *st, const doubl
   const double rr = sum_partials(part_rr, nr, sbuf);
   const double zr = sum_partials(part_zr, nz, sbuf);
   if (threadIdx.x == 0) {
-    if (st->final || st->null_rhs || st->done >= 2) return;
+    if (st->final || st->null_rhs) return;
+    if (st->done >= 2) {
+      // the FP32 iteration broke down inside the chunk (or stopped earlier):
+      // what it left in u is no iterate to keep
+      if (st->done != 2) st->best = 0;
+      return;
+    }
     st->err_true = sqrt(rr) / st->lenf;
     st->rr = rr;
     st->err = st->err_true;
