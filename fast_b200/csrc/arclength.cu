@@ -100,6 +100,7 @@ extern "C" int fast_gpu_arclength_solve(fast_gpu_ctx *c, const double *q_host, c
   const size_t nb = sizeof(double) * n;
   const unsigned G = 148, T = 256;
   Work w;
+  const OnAssembledMatrix on_matrix(*c);
   int rc = FAST_GPU_OK;
   fast_gpu_arc_report R{};
   double lam = 0.0, arclen = 0.0, lenq = 0.0, cf = o->load_coeff, sp0 = 1.0, csp1 = 1.0;

@@ -130,6 +130,8 @@ extern "C" int fast_gpu_autotune(fast_gpu_ctx *c, fast_gpu_tune_report *rep) {
   if (!c || !rep) return FAST_GPU_EINVAL;
   if (!c->K_ok) { c->err = "autotune: matrix not assembled"; return FAST_GPU_ESTATE; }
   fast_gpu_tune_report R{};
+  // the SpMV forms are timed, also inside the iteration: on the assembled matrix
+  const OnAssembledMatrix on_matrix(*c);
 
   // element launch shapes (the timed assemblies add into K; it is rebuilt below)
   bool all_tc = !c->buckets.empty();

@@ -42,6 +42,8 @@ void free_mesh(Ctx &c) {
   c.persist_grid = 0;
   dfree(c.d_lcol);
   dfree(c.d_z2);
+  c.mf.release();
+  c.K_pure = false;
   for (Bucket &B : c.buckets) {
     dfree(B.d_conn); dfree(B.d_E); dfree(B.d_nu); dfree(B.d_rho); dfree(B.d_slot); dfree(B.d_first);
     dfree(B.d_dN); dfree(B.d_N); dfree(B.d_w);
@@ -93,7 +95,7 @@ double *target_of(Ctx &c, int what) {
 }
 
 void invalidate(Ctx &c, int what) {
-  if (what == FAST_ASM_STIFFNESS) { c.Ks_ok = false; c.precond_built = -1; }
+  if (what == FAST_ASM_STIFFNESS) { c.Ks_ok = false; c.precond_built = -1; c.K_pure = false; }
   else c.Ms_ok = false;
 }
 
@@ -256,6 +258,13 @@ int fast_gpu_set_option(fast_gpu_ctx *c, int32_t option, int64_t value) {
     CK(cudaStreamSynchronize(c->stream));
     c->drop_graphs();
     c->use_force_gather = value != 0;
+    return FAST_GPU_OK;
+  }
+  if (option == FAST_OPT_MATRIX_FREE) {
+    if (value < -1) return FAST_GPU_EINVAL;
+    CK(cudaStreamSynchronize(c->stream));
+    c->drop_graphs();
+    c->mf_min_nodes = value;
     return FAST_GPU_OK;
   }
   if (option == FAST_OPT_PERSISTENT_ASSEMBLY) {
@@ -563,6 +572,7 @@ int fast_gpu_pattern_info(fast_gpu_ctx *c, int64_t *nnzb, int64_t *nnz_lower, in
 int fast_gpu_update_coords(fast_gpu_ctx *c, const double *coords) {
   if (check_ctx(c) || !coords || !c->d_X) return FAST_GPU_EINVAL;
   CK(cudaMemcpyAsync(c->d_X, coords, sizeof(double) * 3 * c->nnode, cudaMemcpyHostToDevice, c->stream));
+  c->mf.geo_ok = false;
   c->K_ok = c->M_ok = false;
   invalidate(*c, FAST_ASM_STIFFNESS);
   invalidate(*c, FAST_ASM_MASS);
@@ -599,6 +609,7 @@ int fast_gpu_update_material(fast_gpu_ctx *c, int32_t b, const double *E, const 
     }
     CK(cudaStreamSynchronize(c->stream));
   }
+  c->mf.mat_ok = false;
   c->K_ok = c->M_ok = false;
   invalidate(*c, FAST_ASM_STIFFNESS);
   invalidate(*c, FAST_ASM_MASS);
@@ -685,6 +696,7 @@ int assemble_tf32(fast_gpu_ctx *c) {
     c->err = "assemble: non-positive Jacobian determinant in at least one element";
     return FAST_GPU_EDETJ;
   }
+  c->K_pure = true;
   return FAST_GPU_OK;
 }
 }  // namespace
@@ -712,6 +724,7 @@ int fast_gpu_assemble(fast_gpu_ctx *c, int32_t what) {
     c->err = "assemble: non-positive Jacobian determinant in at least one element";
     return FAST_GPU_EDETJ;
   }
+  if (what == FAST_ASM_STIFFNESS) c->K_pure = true;
   return FAST_GPU_OK;
 }
 
@@ -806,14 +819,22 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
   }
   if (c->precond_built != precond)
     CK(k32 ? launch_build_precond32(*c, c->d_K32, precond) : launch_build_precond(*c, c->d_K, precond));
-  CK(ensure_soa(*c, FAST_ASM_STIFFNESS, mixed));
+  const bool mf = mf_active(*c);
+  c->mf_used = mf;
+  if (mf) {
+    CK(mf_prepare(*c, mixed, precond));
+    if (c->graph_mf_precond != precond) c->drop_graphs();
+    c->graph_mf_precond = precond;
+  } else {
+    CK(ensure_soa(*c, FAST_ASM_STIFFNESS, mixed));
+  }
   const int chunk = opts.check_every > 0 ? opts.check_every : (mixed ? 50 : 32);
   fast_gpu_solve_report R{};
   if (mixed) {
     CK(pcg_mixed(*c, warm, tol, maxit, chunk));
     R.outer = c->h_state->updates;
     int done = c->h_state->done, it = c->h_state->iter;
-    if ((done == 3 || done == 4) && it < maxit && k32) {
+    if ((done == 3 || done == 4) && it < maxit && k32 && !mf) {
       // The tensor-core FP32 stiffness (entries to about 1e-6 of the largest
       // on degree-3 B-splines) could not take this system to the tolerance
       // against its element-by-element FP64 residual, restarts included:
@@ -835,7 +856,7 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
       done = c->h_state->done;
       it = c->h_state->iter;
     }
-    if ((done == 3 || done == 4) && it < maxit && !c->K32_current) {
+    if ((done == 3 || done == 4) && it < maxit && (mf || !c->K32_current)) {
       // FP32 iterates stopped making progress (ill-conditioned system): go on
       // with the FP64 iteration from the best FP64 iterate seen
       R.escalated |= 1;
@@ -1083,6 +1104,12 @@ int fast_gpu_kernel_stats(fast_gpu_ctx *c, int32_t which, int64_t *launches, dou
     if (which == FAST_KERNEL_SPMV_FP32)
       algo = c->spmv32_c16 ? (double)c->nnzb * (9 * 4 + 2) + 4.0 * (c->nnode + 1) + 4.0 * c->nnode + 2.0 * 4 * n4
                            : (double)c->nnzb * (9 * 4 + 4) + 4.0 * (c->nnode + 1) + 2.0 * 4 * n4;
+    // matrix-free solves: incidence, geometry, lambda and mu, the direction (with z) and the element forces once each
+    if (c->mf_used && (which == FAST_KERNEL_SPMV_FP64 || which == FAST_KERNEL_SPMV_FP32)) {
+      const Bucket &B = c->buckets[0];
+      const double t = which == FAST_KERNEL_SPMV_FP64 ? 8.0 : 4.0;
+      algo = (double)B.ne * (4.0 * B.nn + t * (9.0 * B.ng + 2.0 + 3.0 * B.nn)) + 2.0 * t * n4;
+    }
     if (which == FAST_KERNEL_ASSEMBLE || which == FAST_KERNEL_ASSEMBLE_TF32) {
       // scatter model per element: incidence + coordinates + fixity + E, nu + slot map + 3x3 block
       // read-modify-write (72-byte FP64 or 36-byte FP32 blocks), plus the zero fill of the block

@@ -138,6 +138,25 @@ struct TieMaps {
 
 struct PersistPlanHost;  // elem_persist.cu
 
+// Matrix-free operator of one hex bucket (matfree.cu): elements in batches of
+// 32 in the mesh's own order, padded; built at the first solve that uses it
+struct MatFree {
+  bool built = false, geo_ok = false, mat_ok = false, jacobi = true;
+  int nn = 0, nb = 0;              // nodes per element, batches
+  int per_sm32 = 1, per_sm64 = 1;  // resident blocks of the element kernels
+  int32_t *conn = nullptr;         // [nb][nn][32]
+  int32_t *inv = nullptr;          // [ne] colour-sorted position
+  int32_t *ptr = nullptr, *inc = nullptr;  // per node: its entries of F
+  float *g32 = nullptr;            // geometry at the Gauss points
+  double *g64 = nullptr;
+  float2 *lm32 = nullptr;          // [nb][32] lambda, mu
+  double2 *lm64 = nullptr;
+  void *F = nullptr;               // [nb][nn][32][4] element forces, either precision
+  float *dj32 = nullptr;           // [nnode][4] inverse diagonal (Jacobi)
+  double *dj64 = nullptr;
+  void release();
+};
+
 struct Ctx {
   int device = 0;
   cudaStream_t own_stream = nullptr;
@@ -214,6 +233,13 @@ struct Ctx {
   double *d_eq_tmp = nullptr;     // [neq] staging for host <-> device in equation space
   double *h_eq_tmp = nullptr;     // pinned [neq]
 
+  // matrix-free solves (matfree.cu)
+  MatFree mf;
+  bool K_pure = false;           // the stiffness slot is exactly the last small-strain assembly
+  bool mf_off = false;           // a driver that edits or replays the matrix itself is running
+  int64_t mf_min_nodes = -1;     // systems this large take it (-1: the measured default)
+  bool mf_used = false;          // the last solve did
+
   int64_t launches = 0;          // kernels launched by this context (all entry points)
 
   // independent problems in one mesh (fast_gpu_set_problems)
@@ -276,7 +302,14 @@ struct Ctx {
   cudaGraphExec_t graph_fp64 = nullptr, graph_mixed = nullptr;
   int graph_fp64_chunk = 0, graph_mixed_chunk = 0;
   int64_t graph_fp64_kernels = 0, graph_mixed_kernels = 0;
+  // ... of the matrix-free iteration (for one preconditioner)
+  cudaGraphExec_t graph_mf64 = nullptr, graph_mf32 = nullptr;
+  int graph_mf64_chunk = 0, graph_mf32_chunk = 0, graph_mf_precond = -1;
+  int64_t graph_mf64_kernels = 0, graph_mf32_kernels = 0;
   void drop_graphs() {
+    if (graph_mf64) cudaGraphExecDestroy(graph_mf64);
+    if (graph_mf32) cudaGraphExecDestroy(graph_mf32);
+    graph_mf64 = graph_mf32 = nullptr;
     if (graph_fp64) cudaGraphExecDestroy(graph_fp64);
     if (graph_mixed) cudaGraphExecDestroy(graph_mixed);
     graph_fp64 = graph_mixed = nullptr;
@@ -299,6 +332,15 @@ struct Ctx {
   void harvest();                 // closed spans only (call after a stream sync)
 
   bool set_error(const std::string &m) { err = m; return false; }
+};
+
+// No matrix-free solves while a driver runs that edits, times or replays the
+// assembled matrix itself
+struct OnAssembledMatrix {
+  Ctx &c;
+  const bool was;
+  explicit OnAssembledMatrix(Ctx &c_) : c(c_), was(c_.mf_off) { c.mf_off = true; }
+  ~OnAssembledMatrix() { c.mf_off = was; }
 };
 
 // Resident CTAs per SM of one element-kernel launch: the occupancy `occ`,
@@ -409,6 +451,17 @@ cudaError_t launch_matfree_residual(Ctx &c, const double *f, const double *u, do
                                     const int32_t *skip);
 // AoS blocks -> row-local SoA copies (either output may be null)
 cudaError_t launch_to_soa(Ctx &c, const double *K, double *Ks, float *Ks32);
+// matfree.cu: whether the solve of the current stiffness runs matrix-free; its
+// operands (also the preconditioner's compact diagonal); one iteration (dir:
+// the direction is z + beta p, beta from the last update's sums; otherwise p);
+// r = f - K u with r.r in nparts partials, nothing while *skip
+constexpr int64_t kMfNodesHex20 = 65537, kMfNodesHex8 = 65537;
+bool mf_active(const Ctx &c);
+cudaError_t mf_prepare(Ctx &c, bool fp32, int precond);
+template <typename T>
+void mf_iteration(Ctx &c, bool dir, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr);
+cudaError_t mf_residual_of(Ctx &c, const double *f, const double *u, double *r, double *part, int nparts,
+                           const int32_t *skip);
 // PCG on the padded node vectors c.d_f -> c.d_u; state left in c.h_state
 cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int iter0 = 0);
 cudaError_t pcg_mixed(Ctx &c, bool warm, double tol, int maxit, int chunk);

@@ -245,6 +245,7 @@ extern "C" int fast_gpu_nr_solve(fast_gpu_ctx *c, const double *q_host, const fa
   const int32_t n = c->neq;
   const size_t nb = sizeof(double) * n;
   NrWork w;
+  const OnAssembledMatrix on_matrix(*c);
   int rc = FAST_GPU_OK;
   fast_gpu_nr_report R{};
   double lam = 0.0, flen2 = 0.0, rlen2 = 0.0, glen2 = 0.0, best = 0.0;

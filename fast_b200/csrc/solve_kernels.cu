@@ -39,60 +39,9 @@
 #include <cooperative_groups.h>
 
 #include "internal.h"
+#include "solve_common.cuh"
 
 namespace fastgpu {
-
-constexpr int kSpmvThreads = 256;
-constexpr int kVecThreads = 256;
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// block-level fixed-order sum; returns the total in thread 0
-template <int NT>
-__device__ __forceinline__ double block_sum(double v, double *sbuf) {
-  v = warp_sum(v);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sbuf[wid] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x < 32) {
-    t = (lane < NT / 32) ? sbuf[lane] : 0.0;
-    t = warp_sum(t);
-  }
-  return t;
-}
-
-// padded node vectors
-template <typename T> struct V4;
-template <> struct V4<float> {
-  static __device__ __forceinline__ void load(const float *p, float &a, float &b, float &c) {
-    const float4 v = *reinterpret_cast<const float4 *>(p);
-    a = v.x; b = v.y; c = v.z;
-  }
-  static __device__ __forceinline__ void store(float *p, float a, float b, float c) {
-    *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, 0.f);
-  }
-};
-template <> struct V4<double> {
-  static __device__ __forceinline__ void load(const double *p, double &a, double &b, double &c) {
-    const double2 v0 = *reinterpret_cast<const double2 *>(p);
-    a = v0.x; b = v0.y; c = p[2];
-  }
-  static __device__ __forceinline__ void store(double *p, double a, double b, double c) {
-    *reinterpret_cast<double2 *>(p) = make_double2(a, b);
-    *reinterpret_cast<double2 *>(p + 2) = make_double2(c, 0.0);
-  }
-};
 
 // AoS blocks (FP64, or the FP32 tensor-core stiffness) -> padded row-local
 // SoA, FP64 and FP32 copies
@@ -443,21 +392,6 @@ spmv_f64(int64_t nrows, const int32_t *__restrict__ srow, const int32_t *__restr
   }
 }
 
-// single-block fixed-order sum of n partials
-__device__ __forceinline__ double sum_partials(const double *p, int n, double *sbuf) {
-  double v = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) v += p[i];
-  return block_sum<256>(v, sbuf);
-}
-
-// z = Dinv r with Dinv stored as 3 padded rows per node
-template <typename T>
-__device__ __forceinline__ void apply_dinv(const T *D, T r0, T r1, T r2, T &z0, T &z1, T &z2) {
-  z0 = D[0] * r0 + D[1] * r1 + D[2] * r2;
-  z1 = D[4] * r0 + D[5] * r1 + D[6] * r2;
-  z2 = D[8] * r0 + D[9] * r1 + D[10] * r2;
-}
-
 // ---- fused iteration kernels (kernel-per-step path)
 // The scalars of one iteration come from fixed-order sums of per-block
 // partials.  Instead of a single-block kernel between the vector kernels,
@@ -465,20 +399,6 @@ __device__ __forceinline__ void apply_dinv(const T *D, T r0, T r1, T r2, T &z0, 
 // size, same order, hence the same bits) and takes the same decision; the
 // last block to finish (a counter in the state) commits the scalars, so no
 // block ever reads a value another block of the same launch has overwritten.
-
-// true in exactly one thread of the last block to reach this point
-__device__ __forceinline__ bool last_block(uint32_t *counter) {
-  __shared__ bool is_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const uint32_t t = atomicAdd(counter, 1u);
-    is_last = (t == gridDim.x - 1);
-    if (is_last) *counter = 0;
-  }
-  __syncthreads();
-  return is_last && threadIdx.x == 0;
-}
 
 // alpha = dot0 / p.w (every block), then u += alpha p; r -= alpha w;
 // z = Dinv r; partials r.r, z.r.  The last block stores p.w and alpha, or
@@ -1071,7 +991,10 @@ cudaError_t launch_spmv32(Ctx &c, const float *Ks, const float *x, float *y) {
 
 cudaError_t launch_residual(Ctx &c, const double *Ks, const double *f, const double *u, double *r, double *rr_out) {
   double *part = P_E(c);
-  if (Ks) {
+  if (mf_active(c)) {
+    cudaError_t e = mf_residual_of(c, f, u, r, part, spmv_grid(c), nullptr);
+    if (e != cudaSuccess) return e;
+  } else if (Ks) {
     spmv64_go<1>(c, spmv_grid(c), c.nnode, Ks, u, f, r, part, nullptr);
     c.launches++;
   } else {
@@ -2077,7 +2000,9 @@ static void fp64_init(Ctx &c, bool warm, double tol, const double *tol_dev, int 
   const int64_t nn = c.nnode;
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
-  if (warm) {
+  if (warm && mf_active(c)) {
+    mf_residual_of(c, c.d_f, c.d_u, c.d_r, P_E(c), G, nullptr);
+  } else if (warm) {
     spmv64_go<1>(c, G, nn, c.d_Ks, c.d_u, c.d_f, c.d_r, P_E(c), nullptr);
     c.launches++;
   } else {
@@ -2094,6 +2019,12 @@ static void fp64_chunk(Ctx &c, int k) {
   const int64_t nn = c.nnode;
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
+  if (mf_active(c)) {
+    for (int i = 0; i < k; i++) mf_iteration<double>(c, i > 0, c.d_u, c.d_r, c.d_z, c.d_p, P_A(c), P_B(c), P_C(c));
+    pcg_direction_fused<double><<<R, kVecThreads, 0, c.stream>>>(nn, c.d_p, c.d_z, st, P_B(c), P_C(c), R);
+    c.launches++;
+    return;
+  }
   for (int i = 0; i < k; i++) {
     c.begin_span(0);
     spmv64_go<0>(c, G, nn, c.d_Ks, c.d_p, nullptr, c.d_w, P_A(c), &st->done);
@@ -2124,7 +2055,9 @@ static void mixed_reliable(Ctx &c) {
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
   flush_correction<<<R, 256, 0, c.stream>>>(4 * nn, c.d_u, c.s_x, st);
-  if (c.K32_current) {
+  if (mf_active(c)) {
+    mf_residual_of(c, c.d_f, c.d_u, c.d_r, P_E(c), G, &st->final);
+  } else if (c.K32_current) {
     launch_matfree_residual(c, c.d_f, c.d_u, c.d_r, P_E(c), &st->final);  // counts its own launches
   } else {
     c.begin_span(0);
@@ -2146,6 +2079,13 @@ static void mixed_chunk(Ctx &c, int k) {
   const int64_t nn = c.nnode;
   const int G = spmv32_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
+  if (mf_active(c)) {
+    for (int i = 0; i < k; i++) mf_iteration<float>(c, i > 0, c.s_x, c.s_r, c.s_z, c.s_p, P_A(c), P_B(c), P_C(c));
+    pcg_direction_fused<float><<<R, kVecThreads, 0, c.stream>>>(nn, c.s_p, c.s_z, st, P_B(c), P_C(c), R);
+    c.launches++;
+    mixed_reliable(c);
+    return;
+  }
   for (int i = 0; i < k; i++) {
     c.begin_span(1);
     spmv32_go(c, G, nn, c.d_Ks32, c.s_p, c.s_w, P_A(c), &st->done);
@@ -2162,6 +2102,11 @@ cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int it
   cudaError_t e;
   fp64_init(c, warm, tol, nullptr, maxit, iter0);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (mf_active(c))
+    return drive(c, maxit, chunk, &c.graph_mf64, &c.graph_mf64_chunk, &c.graph_mf64_kernels, [&](int k) -> cudaError_t {
+      fp64_chunk(c, k);
+      return cudaGetLastError();
+    });
   if (use_persistent(c)) {
     const int pchunk = chunk < 64 ? 64 : chunk;  // each chunk is one launch: read the state back less often
     return drive(c, maxit, pchunk, nullptr, nullptr, nullptr, [&](int k) -> cudaError_t {
@@ -2180,6 +2125,11 @@ cudaError_t pcg_mixed(Ctx &c, bool warm, double tol, int maxit, int chunk) {
   mixed_init(c, warm, tol, nullptr, maxit);
   mixed_reliable(c);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (mf_active(c))
+    return drive(c, maxit, chunk, &c.graph_mf32, &c.graph_mf32_chunk, &c.graph_mf32_kernels, [&](int k) -> cudaError_t {
+      mixed_chunk(c, k);
+      return cudaGetLastError();
+    });
   if (use_persistent(c)) {
     return drive(c, maxit, chunk, nullptr, nullptr, nullptr, [&](int k) -> cudaError_t {
       cudaError_t el = launch_persistent<float>(c, c.d_Ks32, c.s_x, c.s_r, c.s_z, c.s_p, c.s_p2, c.s_w, c.s_dinv, k);
@@ -2212,7 +2162,7 @@ cudaError_t record_pcg(Ctx &c, bool mixed, bool warm, double tol, const double *
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // small systems iterate in the persistent cooperative kernel (as the
   // launched solves do), a chunk per loop pass
-  const bool persist = use_persistent(c);
+  const bool persist = !mf_active(c) && use_persistent(c);
   // the WHILE node, appended to the graph being captured on c.stream
   cudaStreamCaptureStatus cs;
   cudaGraph_t g = nullptr;

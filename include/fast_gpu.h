@@ -217,6 +217,11 @@ int         fast_gpu_synchronize(fast_gpu_ctx *ctx);
                                             force is formed element by element in one launch per bucket
                                             and gathered per node in the order the colour-by-colour
                                             scatter adds it (the same bits); 0: one launch per colour */
+#define FAST_OPT_MATRIX_FREE         12  /* solves of one small-strain hex8 (2x2x2) or hex20 (3x3x3) bucket
+                                            without ties, on the stiffness as last assembled: from this many
+                                            nodes on K.u is applied element by element instead of by the
+                                            assembled matrix (the same operator to rounding); -1 (default):
+                                            from where it was measured faster */
 #define FAST_OPT_PERSISTENT_ASSEMBLY  8  /* 1: FAST_ASM_STIFFNESS_TF32 integrates the elements of every
                                             bucket in one persistent cooperative launch (colour k of
                                             every bucket is phase k, grid barriers between phases, CTAs
