@@ -819,6 +819,7 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
   }
   if (c->precond_built != precond)
     CK(k32 ? launch_build_precond32(*c, c->d_K32, precond) : launch_build_precond(*c, c->d_K, precond));
+  c->mf_fp32 = mixed;
   const bool mf = mf_active(*c);
   c->mf_used = mf;
   if (mf) {

@@ -146,12 +146,13 @@ struct MatFree {
   int per_sm32 = 1, per_sm64 = 1;  // resident blocks of the element kernels
   int32_t *conn = nullptr;         // [nb][nn][32]
   int32_t *inv = nullptr;          // [ne] colour-sorted position
-  int32_t *ptr = nullptr, *inc = nullptr;  // per node: its entries of F
+  int32_t *ptr = nullptr, *inc = nullptr;  // per node: its entries of F, in fours
   float *g32 = nullptr;            // geometry at the Gauss points
   double *g64 = nullptr;
-  float2 *lm32 = nullptr;          // [nb][32] lambda, mu
-  double2 *lm64 = nullptr;
-  void *F = nullptr;               // [nb][nn][32][4] element forces, either precision
+  float *lam32 = nullptr, *mu32 = nullptr;   // [nb][32]
+  double *lam64 = nullptr, *mu64 = nullptr;
+  float *F32 = nullptr;            // [nb][nn][32][4] element forces and a zero entry
+  double *F64 = nullptr;
   float *dj32 = nullptr;           // [nnode][4] inverse diagonal (Jacobi)
   double *dj64 = nullptr;
   void release();
@@ -238,6 +239,7 @@ struct Ctx {
   bool K_pure = false;           // the stiffness slot is exactly the last small-strain assembly
   bool mf_off = false;           // a driver that edits or replays the matrix itself is running
   int64_t mf_min_nodes = -1;     // systems this large take it (-1: the measured default)
+  bool mf_fp32 = false;          // the solve at hand iterates in FP32
   bool mf_used = false;          // the last solve did
 
   int64_t launches = 0;          // kernels launched by this context (all entry points)
@@ -452,14 +454,14 @@ cudaError_t launch_matfree_residual(Ctx &c, const double *f, const double *u, do
 // AoS blocks -> row-local SoA copies (either output may be null)
 cudaError_t launch_to_soa(Ctx &c, const double *K, double *Ks, float *Ks32);
 // matfree.cu: whether the solve of the current stiffness runs matrix-free; its
-// operands (also the preconditioner's compact diagonal); one iteration (dir:
-// the direction is z + beta p, beta from the last update's sums; otherwise p);
-// r = f - K u with r.r in nparts partials, nothing while *skip
-constexpr int64_t kMfNodesHex20 = 65537, kMfNodesHex8 = 65537;
+// operands (also the preconditioner's compact diagonal); k iterations from the
+// direction p (pcg_direction_fused has to follow: the last update's sums are in
+// part_rr and part_zr); r = f - K u with r.r in nparts partials, nothing while
+// *skip
 bool mf_active(const Ctx &c);
 cudaError_t mf_prepare(Ctx &c, bool fp32, int precond);
 template <typename T>
-void mf_iteration(Ctx &c, bool dir, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr);
+void mf_iterations(Ctx &c, int k, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr);
 cudaError_t mf_residual_of(Ctx &c, const double *f, const double *u, double *r, double *part, int nparts,
                            const int32_t *skip);
 // PCG on the padded node vectors c.d_f -> c.d_u; state left in c.h_state

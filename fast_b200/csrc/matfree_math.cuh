@@ -14,6 +14,10 @@
 //   G = H A (H_cd = du_c/dxi_d), S = lambda tr(G) I + mu (G + G^T), P = S A^T,
 // and P goes back through the transposes.  Node numbering: FAST's local order
 // (hex8 shp/shpsolid.cpp:173-184, hex20 :301-325).
+//
+// The hex20 steps carry a factor of 8 (kScale20), which removes every
+// halving: H comes out 8 times too large, the transposes return another 8, and
+// lambda and mu are taken divided by 64 (exact).
 #pragma once
 
 #ifdef __CUDACC__
@@ -25,140 +29,171 @@
 namespace fastgpu {
 namespace mf {
 
+template <typename T>
+FG_HD T mad(T a, T b, T c) {
+  return a * b + c;
+}
+
 // hex20: vertical edge i (corner (-,-), (+,-), (+,+), (-,+)): nodes at z = 1, -1, 0;
 // mid i ((0,-), (+,0), (0,+), (-,0)): nodes at z = 1, -1; it lies between corners i and i + 1
-FG_HD int corner_top(int i) { return 2 * i; }
-FG_HD int corner_bot(int i) { return 12 + 2 * i; }
-FG_HD int corner_mid(int i) { return 8 + i; }
-FG_HD int mid_top(int i) { return 1 + 2 * i; }
-FG_HD int mid_bot(int i) { return 13 + 2 * i; }
+FG_HD constexpr int corner_top(int i) { return 2 * i; }
+FG_HD constexpr int corner_bot(int i) { return 12 + 2 * i; }
+FG_HD constexpr int corner_mid(int i) { return 8 + i; }
+FG_HD constexpr int mid_top(int i) { return 1 + 2 * i; }
+FG_HD constexpr int mid_bot(int i) { return 13 + 2 * i; }
 
 constexpr double kA20 = 0.77459666924148337704;  // sqrt(0.6): the 3-point Gauss abscissa
 constexpr double kA8 = 0.57735026918962576451;   // sqrt(1/3)
+constexpr double kScale20 = 8.0;
 
-// coefficients of the 8-node serendipity polynomial from the values at the
-// corners c and mids m; k: x, y, xx, yy, xy, xxy, xyy, 1
+// The 8-node serendipity polynomial k of values c (corners) and m (mids), from
+// C = 2 c, M = 2 m: 8 k of x: A - w, y: B2 - v, xy: B, xx: u, xxy: v, yy: s, xyy: w, 1: e - s
 template <typename T>
-FG_HD void face_poly(const T *c, const T *m, T *k) {
-  const T h = T(0.5);
-  const T q1 = h * (c[0] + c[1]) - m[0], q2 = h * (c[1] + c[2]) - m[1], q3 = h * (c[2] + c[3]) - m[2],
-          q4 = h * (c[3] + c[0]) - m[3];
-  const T s1 = h * (c[1] - c[0]), s3 = h * (c[2] - c[3]), t4 = h * (c[3] - c[0]), t2 = h * (c[2] - c[1]);
-  k[2] = h * (q1 + q3);
-  k[5] = h * (q3 - q1);
-  k[3] = h * (q2 + q4);
-  k[6] = h * (q2 - q4);
-  k[4] = h * (s3 - s1);
-  k[0] = h * (s1 + s3) - k[6];
-  k[1] = h * (t4 + t2) - k[5];
-  k[7] = h * (m[0] + m[2]) - k[3];
+struct Face {
+  T A, B, B2, u, v, s, w;
+};
+template <typename T>
+FG_HD Face<T> face_poly(const T *C, const T *M) {
+  const T two = T(-2.0);
+  const T q1 = mad(two, M[0], C[0] + C[1]), q2 = mad(two, M[1], C[1] + C[2]), q3 = mad(two, M[2], C[2] + C[3]),
+          q4 = mad(two, M[3], C[3] + C[0]);
+  const T p = C[1] - C[0], r = C[2] - C[3];
+  return {p + r, r - p, (C[3] - C[0]) + (C[2] - C[1]), q1 + q3, q3 - q1, q2 + q4, q2 - q4};
+}
+// transpose: the adjoints of the seven -> C, M
+template <typename T>
+FG_HD void face_poly_t(const Face<T> &F, T *C, T *M) {
+  const T two = T(-2.0);
+  const T q1 = F.u - F.v, q3 = F.u + F.v, q2 = F.s + F.w, q4 = F.s - F.w;
+  const T p = F.A - F.B, r = F.A + F.B, t = F.B2;
+  const T pm = p + t, pp = p - t, rp = r + t, rm = t - r;
+  C[0] = (q1 + q4) - pm;
+  C[1] = (q1 + q2) + pp;
+  C[2] = (q2 + q3) + rp;
+  C[3] = (q3 + q4) + rm;
+  M[0] = two * q1;
+  M[1] = two * q2;
+  M[2] = two * q3;
+  M[3] = two * q4;
 }
 
-// transpose: k (overwritten) -> c, m; with_one: k[7] takes part
+// Planes z = (k - 1) sqrt(0.6) and lines y = (j - 1) sqrt(0.6) are taken by
+// their coordinates, not as template parameters: one copy of the code for all
+// (three unrolled copies of the planes overran the instruction cache).
 template <typename T>
-FG_HD void face_poly_t(T *k, bool with_one, T *c, T *m) {
-  const T h = T(0.5);
-  T one = T(0);
-  if (with_one) {
-    one = h * k[7];
-    k[3] -= k[7];
-  }
-  k[6] -= k[0];
-  k[5] -= k[1];
-  const T s1 = h * (k[0] - k[4]), s3 = h * (k[0] + k[4]), t = h * k[1];
-  const T q1 = h * (k[2] - k[5]), q3 = h * (k[2] + k[5]), q4 = h * (k[3] - k[6]), q2 = h * (k[3] + k[6]);
-  c[0] = h * (q1 + q4 - s1 - t);
-  c[1] = h * (q1 + q2 + s1 - t);
-  c[2] = h * (q3 + q2 + s3 + t);
-  c[3] = h * (q3 + q4 - s3 + t);
-  m[0] = one - q1;
-  m[1] = -q2;
-  m[2] = one - q3;
-  m[3] = -q4;
+FG_HD T gauss20(int k) {
+  return k == 0 ? T(-kA20) : (k == 1 ? T(0.0) : T(kA20));
+}
+template <typename T>
+FG_HD T gauss20_sq(int k) {
+  return k == 1 ? T(0.0) : T(0.6);
 }
 
-// one component of a hex20 field on the plane z = (k - 1) sqrt(0.6): the 8
-// line coefficients of each of its lines y = (j - 1) sqrt(0.6),
-//   d/dx = L0 + L1 x, d/dy = L2 + L3 x + L4 x^2, d/dz = L5 + L6 x + L7 x^2
+// one component of a hex20 field on the plane z (zz = z^2): its polynomial
+// there (p) and that of its z derivative (q; d0, dy: constant and y)
 template <typename T>
-FG_HD void plane_lines(const T *f, int k, T (*L)[8]) {
-  const T a = T(kA20), h = T(0.5), z = k == 0 ? -a : (k == 1 ? T(0) : a), zz = k == 1 ? T(0) : T(0.6);
-  T d[4], c[4], m[4], cz[4], mz[4];
+struct Plane {
+  Face<T> p, q;
+  T d0, dy;
+};
+template <typename T>
+FG_HD Plane<T> plane_poly(const T *f, T z, T zz) {
+  const T z2 = z + z, g = T(0.5) * zz - T(0.5);
+  T D[4], C[4], M[4], CZ[4], MZ[4];
+#ifdef __CUDACC__
+#pragma unroll
+#endif
   for (int i = 0; i < 4; i++) {
     const T fp = f[corner_top(i)], fm = f[corner_bot(i)], f0 = f[corner_mid(i)];
-    const T o = h * (fp - fm);
-    d[i] = h * (fp + fm) - f0;
-    c[i] = f0 + z * o + zz * d[i];
-    cz[i] = o + T(2) * z * d[i];
+    const T O = fp - fm, F = f0 + f0;
+    D[i] = (fp + fm) - F;
+    C[i] = mad(z, O, mad(zz, D[i], F));
+    CZ[i] = mad(z2, D[i], O);
   }
+#ifdef __CUDACC__
+#pragma unroll
+#endif
   for (int i = 0; i < 4; i++) {
     const T fp = f[mid_top(i)], fm = f[mid_bot(i)];
-    const T o = h * (fp - fm), e = h * (fp + fm), g = h * (d[i] + d[(i + 1) & 3]);
-    m[i] = e + z * o - (T(1) - zz) * g;
-    mz[i] = o + T(2) * z * g;
+    const T O = fp - fm, G = D[i] + D[(i + 1) & 3];
+    M[i] = mad(z, O, mad(g, G, fp + fm));
+    MZ[i] = mad(z, G, O);
   }
-  T p[8], q[8];
-  face_poly(c, m, p);
-  face_poly(cz, mz, q);
-  for (int j = 0; j < 3; j++) {
-    const T y = j == 0 ? -a : (j == 1 ? T(0) : a), yy = j == 1 ? T(0) : T(0.6);
-    L[j][0] = p[0] + y * p[4] + yy * p[6];
-    L[j][1] = T(2) * (p[2] + y * p[5]);
-    L[j][2] = p[1] + T(2) * y * p[3];
-    L[j][3] = p[4] + T(2) * y * p[6];
-    L[j][4] = p[5];
-    L[j][5] = q[7] + y * q[1] + yy * q[3];
-    L[j][6] = q[0] + y * q[4] + yy * q[6];
-    L[j][7] = q[2] + y * q[5];
-  }
+  Plane<T> P;
+  P.p = face_poly(C, M);
+  P.q = face_poly(CZ, MZ);
+  P.d0 = mad(T(2.0), MZ[0] + MZ[2], -P.q.s);
+  P.dy = P.q.B2 - P.q.v;
+  return P;
+}
+// the 8 line coefficients on y (yy = y^2), scaled by 8:
+//   d/dx = L0 + 2 x L1, d/dy = L2 + x L3 + x^2 L4, d/dz = L5 + x L6 + x^2 L7
+template <typename T>
+FG_HD void plane_line(const Plane<T> &P, T y, T yy, T *L) {
+  const T y2 = y + y, c = yy - T(1.0);
+  L[0] = mad(y, P.p.B, mad(c, P.p.w, P.p.A));
+  L[1] = mad(y, P.p.v, P.p.u);
+  L[2] = mad(y2, P.p.s, P.p.B2 - P.p.v);
+  L[3] = mad(y2, P.p.w, P.p.B);
+  L[4] = P.p.v;
+  L[5] = mad(y, P.dy, mad(yy, P.q.s, P.d0));
+  L[6] = mad(y, P.q.B, mad(c, P.q.w, P.q.A));
+  L[7] = mad(y, P.q.v, P.q.u);
 }
 
-// transpose: the plane's line coefficients -> its part of the nodal values
+// transposes.  A line's results R are added to the plane's adjoint N (zeroed
+// before), whose p.A ... q.w, d0 and dy are the adjoints of the plane's ...
 template <typename T>
-FG_HD void plane_lines_t(const T (*L)[8], int k, T *f) {
-  const T a = T(kA20), h = T(0.5), z = k == 0 ? -a : (k == 1 ? T(0) : a), zz = k == 1 ? T(0) : T(0.6);
-  const T b = T(0.6);
-  T p[8], q[8], c[4], m[4], cz[4], mz[4];
-  {
-    const T s0 = L[0][0] + L[2][0], d0 = a * (L[2][0] - L[0][0]);
-    const T s1 = L[0][1] + L[2][1], d1 = a * (L[2][1] - L[0][1]);
-    const T s2 = L[0][2] + L[2][2], d2 = a * (L[2][2] - L[0][2]);
-    const T s3 = L[0][3] + L[2][3], d3 = a * (L[2][3] - L[0][3]);
-    p[0] = s0 + L[1][0];
-    p[4] = d0 + s3 + L[1][3];
-    p[6] = b * s0 + T(2) * d3;
-    p[2] = T(2) * (s1 + L[1][1]);
-    p[5] = T(2) * d1 + (L[0][4] + L[1][4] + L[2][4]);
-    p[1] = s2 + L[1][2];
-    p[3] = T(2) * d2;
-    p[7] = T(0);
-  }
-  {
-    const T s0 = L[0][5] + L[2][5], s1 = L[0][6] + L[2][6], s2 = L[0][7] + L[2][7];
-    q[7] = s0 + L[1][5];
-    q[1] = a * (L[2][5] - L[0][5]);
-    q[3] = b * s0;
-    q[0] = s1 + L[1][6];
-    q[4] = a * (L[2][6] - L[0][6]);
-    q[6] = b * s1;
-    q[2] = s2 + L[1][7];
-    q[5] = a * (L[2][7] - L[0][7]);
-  }
-  face_poly_t(p, false, c, m);
-  face_poly_t(q, true, cz, mz);
-  T g[4];
+FG_HD void plane_line_t(const T *R, T y, T yy, Plane<T> &N) {
+  const T y2 = y + y, c = yy - T(1.0);
+  N.p.A += R[0];
+  N.p.B += mad(y, R[0], R[3]);
+  N.p.w += mad(c, R[0], y2 * R[3]);
+  N.p.u += R[1];
+  N.p.v += mad(y, R[1], R[4] - R[2]);
+  N.p.B2 += R[2];
+  N.p.s = mad(y2, R[2], N.p.s);
+  N.d0 += R[5];
+  N.dy = mad(y, R[5], N.dy);
+  N.q.s = mad(yy, R[5], N.q.s);
+  N.q.A += R[6];
+  N.q.B = mad(y, R[6], N.q.B);
+  N.q.w = mad(c, R[6], N.q.w);
+  N.q.u += R[7];
+  N.q.v = mad(y, R[7], N.q.v);
+}
+// ... and the plane's adjoint goes to its part of the nodal values
+template <typename T>
+FG_HD void plane_poly_t(Plane<T> &N, T z, T zz, T *f) {
+  const T z2 = z + z, g = T(0.5) * zz - T(0.5);
+  T C[4], M[4], CZ[4], MZ[4];
+  N.q.B2 = N.dy;
+  N.q.v -= N.dy;
+  N.q.s -= N.d0;
+  face_poly_t(N.p, C, M);
+  face_poly_t(N.q, CZ, MZ);
+  MZ[0] = mad(T(2.0), N.d0, MZ[0]);
+  MZ[2] = mad(T(2.0), N.d0, MZ[2]);
+  T G[4];
+#ifdef __CUDACC__
+#pragma unroll
+#endif
   for (int i = 0; i < 4; i++) {
-    const T o = z * m[i] + mz[i];
-    g[i] = T(2) * z * mz[i] - (T(1) - zz) * m[i];
-    f[mid_top(i)] = h * (m[i] + o);
-    f[mid_bot(i)] = h * (m[i] - o);
+    const T O = mad(z, M[i], MZ[i]);
+    G[i] = mad(z, MZ[i], g * M[i]);
+    f[mid_top(i)] = M[i] + O;
+    f[mid_bot(i)] = M[i] - O;
   }
+#ifdef __CUDACC__
+#pragma unroll
+#endif
   for (int i = 0; i < 4; i++) {
-    const T o = z * c[i] + cz[i];
-    const T d = zz * c[i] + T(2) * z * cz[i] + h * (g[i] + g[(i + 3) & 3]);
-    f[corner_top(i)] = h * (d + o);
-    f[corner_bot(i)] = h * (d - o);
-    f[corner_mid(i)] = c[i] - d;
+    const T O = mad(z, C[i], CZ[i]);
+    const T D = mad(zz, C[i], mad(z2, CZ[i], G[i] + G[(i + 3) & 3]));
+    f[corner_top(i)] = D + O;
+    f[corner_bot(i)] = D - O;
+    const T m = C[i] - D;
+    f[corner_mid(i)] = m + m;
   }
 }
 
@@ -166,95 +201,125 @@ FG_HD void plane_lines_t(const T (*L)[8], int k, T *f) {
 template <typename T>
 FG_HD void point_stress(const T *H, const T *A, T lam, T mu, T *P) {
   T G[9];
+#ifdef __CUDACC__
+#pragma unroll
+#endif
   for (int c = 0; c < 3; c++)
-    for (int j = 0; j < 3; j++) G[3 * c + j] = H[3 * c] * A[j] + H[3 * c + 1] * A[3 + j] + H[3 * c + 2] * A[6 + j];
-  const T tr = lam * (G[0] + G[4] + G[8]);
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+    for (int j = 0; j < 3; j++) G[3 * c + j] = mad(H[3 * c], A[j], mad(H[3 * c + 1], A[3 + j], H[3 * c + 2] * A[6 + j]));
+  const T tr = lam * ((G[0] + G[4]) + G[8]);
   const T m2 = mu + mu;
-  const T s0 = tr + m2 * G[0], s1 = tr + m2 * G[4], s2 = tr + m2 * G[8];
+  const T s0 = mad(m2, G[0], tr), s1 = mad(m2, G[4], tr), s2 = mad(m2, G[8], tr);
   const T s01 = mu * (G[1] + G[3]), s02 = mu * (G[2] + G[6]), s12 = mu * (G[5] + G[7]);
+#ifdef __CUDACC__
+#pragma unroll
+#endif
   for (int d = 0; d < 3; d++) {
     const T a0 = A[3 * d], a1 = A[3 * d + 1], a2 = A[3 * d + 2];
-    P[d] = s0 * a0 + s01 * a1 + s02 * a2;
-    P[3 + d] = s01 * a0 + s1 * a1 + s12 * a2;
-    P[6 + d] = s02 * a0 + s12 * a1 + s2 * a2;
+    P[d] = mad(s0, a0, mad(s01, a1, s02 * a2));
+    P[3 + d] = mad(s01, a0, mad(s1, a1, s12 * a2));
+    P[6 + d] = mad(s02, a0, mad(s12, a1, s2 * a2));
   }
 }
 
-// a line's three points: L[c][8] (overwritten with the transposed result),
-// geometry A(i, q) of point i
-template <typename T, typename Geo>
-FG_HD void line_points(T (*L)[8], const Geo &A, T lam, T mu) {
-  const T a = T(kA20);
-  T R[3][8];
-  for (int c = 0; c < 3; c++)
-    for (int q = 0; q < 8; q++) R[c][q] = T(0);
-  for (int i = 0; i < 3; i++) {
-    const T x = i == 0 ? -a : (i == 1 ? T(0) : a), xx = i == 1 ? T(0) : T(0.6);
-    T H[9], P[9], Ag[9];
-    for (int q = 0; q < 9; q++) Ag[q] = A(i, q);
-    for (int c = 0; c < 3; c++) {
-      H[3 * c] = L[c][0] + x * L[c][1];
-      H[3 * c + 1] = L[c][2] + x * L[c][3] + xx * L[c][4];
-      H[3 * c + 2] = L[c][5] + x * L[c][6] + xx * L[c][7];
-    }
-    point_stress(H, Ag, lam, mu, P);
-    for (int c = 0; c < 3; c++) {
-      R[c][0] += P[3 * c];
-      R[c][1] += x * P[3 * c];
-      R[c][2] += P[3 * c + 1];
-      R[c][3] += x * P[3 * c + 1];
-      R[c][4] += xx * P[3 * c + 1];
-      R[c][5] += P[3 * c + 2];
-      R[c][6] += x * P[3 * c + 2];
-      R[c][7] += xx * P[3 * c + 2];
-    }
+// a line's gradients at its three points x = -sqrt(0.6), 0, sqrt(0.6):
+// L[c][8] -> H[point][3 c + d], and the transpose.  (All three at once, P in
+// H's place afterwards: the line's 24 coefficients are dead while the points
+// are worked on.)
+template <typename T>
+FG_HD void line_gradients(const T (*L)[8], T (*H)[9]) {
+  const T a = T(kA20), na = T(-kA20), a2 = T(2 * kA20), na2 = T(-2 * kA20), b = T(0.6);
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+  for (int c = 0; c < 3; c++) {
+    H[0][3 * c] = mad(na2, L[c][1], L[c][0]);
+    H[1][3 * c] = L[c][0];
+    H[2][3 * c] = mad(a2, L[c][1], L[c][0]);
+    const T y = mad(b, L[c][4], L[c][2]), z = mad(b, L[c][7], L[c][5]);
+    H[0][3 * c + 1] = mad(na, L[c][3], y);
+    H[1][3 * c + 1] = L[c][2];
+    H[2][3 * c + 1] = mad(a, L[c][3], y);
+    H[0][3 * c + 2] = mad(na, L[c][6], z);
+    H[1][3 * c + 2] = L[c][5];
+    H[2][3 * c + 2] = mad(a, L[c][6], z);
   }
-  for (int c = 0; c < 3; c++)
-    for (int q = 0; q < 8; q++) L[c][q] = R[c][q];
+}
+template <typename T>
+FG_HD void line_gradients_t(const T (*P)[9], T (*R)[8]) {
+  const T a = T(kA20), a2 = T(2 * kA20), b = T(0.6);
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+  for (int c = 0; c < 3; c++) {
+    R[c][0] = (P[0][3 * c] + P[2][3 * c]) + P[1][3 * c];
+    R[c][1] = a2 * (P[2][3 * c] - P[0][3 * c]);
+    const T y = P[0][3 * c + 1] + P[2][3 * c + 1], z = P[0][3 * c + 2] + P[2][3 * c + 2];
+    R[c][2] = y + P[1][3 * c + 1];
+    R[c][3] = a * (P[2][3 * c + 1] - P[0][3 * c + 1]);
+    R[c][4] = b * y;
+    R[c][5] = z + P[1][3 * c + 2];
+    R[c][6] = a * (P[2][3 * c + 2] - P[0][3 * c + 2]);
+    R[c][7] = b * z;
+  }
 }
 
 // hex8, one component: nodal values -> the derivatives, each of which is
 // constant along its own direction: D[0] = d/dx at (y, z) signs 2 bits
 // (y + 2 z), D[1] = d/dy at x + 2 z, D[2] = d/dz at x + 2 y
 template <typename T>
+FG_HD void four_signs(T c, T u, T v, T uv, T *out) {  // c +- u +- v +- uv
+  const T a = c - v, b = c + v, d = u - uv, e = u + uv;
+  out[0] = a - d;
+  out[1] = a + d;
+  out[2] = b - e;
+  out[3] = b + e;
+}
+template <typename T>
+FG_HD void four_signs_t(const T *in, T &c, T &u, T &v, T &uv) {
+  const T a = in[0] + in[1], b = in[2] + in[3], d = in[1] - in[0], e = in[3] - in[2];
+  c = a + b;
+  u = d + e;
+  v = b - a;
+  uv = e - d;
+}
+template <typename T>
 FG_HD void hex8_grads(const T *f, T (*D)[4]) {
   // corner pairs of FAST's order: nodes 0..3 at z = 1: (-,-) (+,-) (+,+) (-,+); 4..7 at z = -1
   const T w = T(0.125), s = T(0.125 * kA8), t = T(0.125 / 3.0);
   T e[4], o[4];
-  for (int i = 0; i < 4; i++) { e[i] = f[i] + f[4 + i]; o[i] = f[i] - f[4 + i]; }
-  const T ex = (e[1] - e[0]) + (e[2] - e[3]), exy = (e[0] - e[1]) + (e[2] - e[3]),
-          ey = (e[2] - e[1]) + (e[3] - e[0]);
-  const T o0 = (o[0] + o[1]) + (o[2] + o[3]), ox = (o[1] - o[0]) + (o[2] - o[3]),
-          oxy = (o[0] - o[1]) + (o[2] - o[3]), oy = (o[2] - o[1]) + (o[3] - o[0]);
-  auto four = [](T c, T u, T v, T uv, T *out) {  // c +- u +- v +- uv
-    out[0] = (c - u) - (v - uv);
-    out[1] = (c + u) - (v + uv);
-    out[2] = (c - u) + (v - uv);
-    out[3] = (c + u) + (v + uv);
-  };
-  four(w * ex, s * exy, s * ox, t * oxy, D[0]);   // u: y, v: z
-  four(w * ey, s * exy, s * oy, t * oxy, D[1]);   // u: x, v: z
-  four(w * o0, s * ox, s * oy, t * oxy, D[2]);    // u: x, v: y
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+  for (int i = 0; i < 4; i++) {
+    e[i] = f[i] + f[4 + i];
+    o[i] = f[i] - f[4 + i];
+  }
+  const T ep = e[1] - e[0], er = e[2] - e[3], op = o[1] - o[0], orr = o[2] - o[3];
+  const T ex = ep + er, exy = er - ep, ey = (e[2] - e[1]) + (e[3] - e[0]);
+  const T o0 = (o[0] + o[1]) + (o[2] + o[3]), ox = op + orr, oxy = orr - op, oy = (o[2] - o[1]) + (o[3] - o[0]);
+  const T se = s * exy, sx = s * ox, sy = s * oy, tt = t * oxy;
+  four_signs(w * ex, se, sx, tt, D[0]);   // u: y, v: z
+  four_signs(w * ey, se, sy, tt, D[1]);   // u: x, v: z
+  four_signs(w * o0, sx, sy, tt, D[2]);   // u: x, v: y
 }
 template <typename T>
 FG_HD void hex8_grads_t(const T (*D)[4], T *f) {
   const T w = T(0.125), s = T(0.125 * kA8), t = T(0.125 / 3.0);
-  auto four = [](const T *in, T &c, T &u, T &v, T &uv) {
-    const T a = in[0] + in[1], b = in[2] + in[3], d = in[1] - in[0], e = in[3] - in[2];
-    c = a + b;
-    u = d + e;
-    v = b - a;
-    uv = e - d;
-  };
   T c0, u0, v0, w0, c1, u1, v1, w1, c2, u2, v2, w2;
-  four(D[0], c0, u0, v0, w0);
-  four(D[1], c1, u1, v1, w1);
-  four(D[2], c2, u2, v2, w2);
-  const T ex = w * c0, exy = s * (u0 + u1), ox = s * (v0 + u2), oxy = t * (w0 + w1 + w2), ey = w * c1,
+  four_signs_t(D[0], c0, u0, v0, w0);
+  four_signs_t(D[1], c1, u1, v1, w1);
+  four_signs_t(D[2], c2, u2, v2, w2);
+  const T ex = w * c0, exy = s * (u0 + u1), ox = s * (v0 + u2), oxy = t * ((w0 + w1) + w2), ey = w * c1,
           oy = s * (v1 + v2), o0 = w * c2;
-  const T e[4] = {-ex + exy - ey, ex - exy - ey, ex + exy + ey, -ex - exy + ey};
-  const T o[4] = {o0 - ox + oxy - oy, o0 + ox - oxy - oy, o0 + ox + oxy + oy, o0 - ox - oxy + oy};
-  for (int i = 0; i < 4; i++) { f[i] = e[i] + o[i]; f[4 + i] = e[i] - o[i]; }
+  const T exa = ex + exy, exb = ex - exy, oxa = ox + oxy, oxb = ox - oxy;
+  const T e0 = T(-1.0) * (exb + ey), e1 = exb - ey, e2 = exa + ey, e3 = ey - exa;
+  const T oa = o0 - oy, ob = o0 + oy;
+  const T q0 = oa - oxb, q1 = oa + oxb, q2 = ob + oxa, q3 = ob - oxa;
+  f[0] = e0 + q0; f[1] = e1 + q1; f[2] = e2 + q2; f[3] = e3 + q3;
+  f[4] = e0 - q0; f[5] = e1 - q1; f[6] = e2 - q2; f[7] = e3 - q3;
 }
 
 }  // namespace mf

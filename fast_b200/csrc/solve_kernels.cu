@@ -2020,7 +2020,7 @@ static void fp64_chunk(Ctx &c, int k) {
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
   if (mf_active(c)) {
-    for (int i = 0; i < k; i++) mf_iteration<double>(c, i > 0, c.d_u, c.d_r, c.d_z, c.d_p, P_A(c), P_B(c), P_C(c));
+    mf_iterations<double>(c, k, c.d_u, c.d_r, c.d_z, c.d_p, P_A(c), P_B(c), P_C(c));
     pcg_direction_fused<double><<<R, kVecThreads, 0, c.stream>>>(nn, c.d_p, c.d_z, st, P_B(c), P_C(c), R);
     c.launches++;
     return;
@@ -2080,7 +2080,7 @@ static void mixed_chunk(Ctx &c, int k) {
   const int G = spmv32_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
   if (mf_active(c)) {
-    for (int i = 0; i < k; i++) mf_iteration<float>(c, i > 0, c.s_x, c.s_r, c.s_z, c.s_p, P_A(c), P_B(c), P_C(c));
+    mf_iterations<float>(c, k, c.s_x, c.s_r, c.s_z, c.s_p, P_A(c), P_B(c), P_C(c));
     pcg_direction_fused<float><<<R, kVecThreads, 0, c.stream>>>(nn, c.s_p, c.s_z, st, P_B(c), P_C(c), R);
     c.launches++;
     mixed_reliable(c);
