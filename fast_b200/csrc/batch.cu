@@ -4,7 +4,8 @@
 // (mlib/sysmat.cpp:1061-1125) stopping test.  The meshes are uploaded as one
 // mesh with disjoint node ranges, so assembly, the block pattern and the
 // solve layout are those of a single system whose matrix is block diagonal;
-// the solve runs one CTA per problem in a single launch.
+// the solve runs all problems at once, matrix-free an iteration at a time
+// (matfree.cu) or a cluster of blocks per problem in a single launch (pcg_batch).
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -29,6 +30,9 @@ void free_problems(Ctx &c) {
   c.d_perr = nullptr;
   c.nprob = 0;
   c.h_noff.clear();
+  c.h_order.clear();
+  c.drop_graphs();
+  c.mf.release();  // (its batches follow the problems)
 }
 
 }  // namespace
@@ -79,6 +83,7 @@ extern "C" int fast_gpu_set_problems(fast_gpu_ctx *c, int32_t num_problems, cons
   BCK(cudaMemcpy(c->d_order, order.data(), sizeof(int32_t) * num_problems, cudaMemcpyHostToDevice));
   c->nprob = num_problems;
   c->h_noff = off;
+  c->h_order = order;
   return FAST_GPU_OK;
 }
 
@@ -99,7 +104,9 @@ extern "C" int fast_gpu_solve_batch(fast_gpu_ctx *c, const double *f, double *u,
   for (int k = 0; k < c->nprob; k++) biggest = std::max(biggest, c->h_noff[k + 1] - c->h_noff[k]);
   const int maxit = opts.maxit > 0 ? opts.maxit : (int)std::max<int64_t>(60 * biggest, 100);
   if (c->precond_built != opts.precond) BCK(launch_build_precond(*c, c->d_K, opts.precond));
-  BCK(solve_layout(*c, FAST_ASM_STIFFNESS, false));
+  const bool mf = mf_batch_active(*c);
+  if (mf) BCK(mf_prepare(*c, false, opts.precond));
+  else BCK(solve_layout(*c, FAST_ASM_STIFFNESS, false));
   const size_t nb = sizeof(double) * c->neq;
   BCK(cudaMemcpyAsync(c->d_eq_tmp, f, nb, cudaMemcpyHostToDevice, c->stream));
   BCK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_f));
@@ -108,16 +115,20 @@ extern "C" int fast_gpu_solve_batch(fast_gpu_ctx *c, const double *f, double *u,
     BCK(cudaMemcpyAsync(c->d_eq_tmp, u, nb, cudaMemcpyHostToDevice, c->stream));
     BCK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_u));
   }
+  std::vector<int32_t> it(c->nprob), dn(c->nprob);
+  std::vector<double> er(c->nprob);
   const int64_t sp = c->begin_span(FAST_KERNEL_LINEAR_SOLVE);
-  BCK(launch_pcg_batch(*c, c->nprob, c->d_order, c->d_noff, tol, maxit, warm, c->d_piters, c->d_perr, c->d_pdone));
+  if (mf) {
+    BCK(mf_solve_batch(*c, tol, maxit, warm, it.data(), er.data(), dn.data()));
+  } else {
+    BCK(launch_pcg_batch(*c, c->nprob, c->d_order, c->d_noff, tol, maxit, warm, c->d_piters, c->d_perr, c->d_pdone));
+    BCK(cudaMemcpyAsync(it.data(), c->d_piters, sizeof(int32_t) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
+    BCK(cudaMemcpyAsync(dn.data(), c->d_pdone, sizeof(int32_t) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
+    BCK(cudaMemcpyAsync(er.data(), c->d_perr, sizeof(double) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
+  }
   c->end_span(sp);
   BCK(launch_node_to_eq(*c, c->d_u, c->d_eq_tmp));
   BCK(cudaMemcpyAsync(u, c->d_eq_tmp, nb, cudaMemcpyDeviceToHost, c->stream));
-  std::vector<int32_t> it(c->nprob), dn(c->nprob);
-  std::vector<double> er(c->nprob);
-  BCK(cudaMemcpyAsync(it.data(), c->d_piters, sizeof(int32_t) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
-  BCK(cudaMemcpyAsync(dn.data(), c->d_pdone, sizeof(int32_t) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
-  BCK(cudaMemcpyAsync(er.data(), c->d_perr, sizeof(double) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
   BCK(cudaStreamSynchronize(c->stream));
   c->harvest();
   int bad = 0;

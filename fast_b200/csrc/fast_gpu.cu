@@ -79,6 +79,7 @@ void free_mesh(Ctx &c) {
   c.d_noff = nullptr; c.d_order = nullptr; c.d_piters = nullptr; c.d_pdone = nullptr; c.d_perr = nullptr;
   c.nprob = 0;
   c.h_noff.clear();
+  c.h_order.clear();
   c.nnode = 0;
   c.neq = 0;
   c.nnzb = 0;

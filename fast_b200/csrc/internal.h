@@ -138,6 +138,12 @@ struct TieMaps {
 
 struct PersistPlanHost;  // elem_persist.cu
 
+// PCG state of one of many independent problems (matfree.cu)
+struct MfProblem {
+  double lenf, dot0, beta, alpha, err;
+  int32_t iter, done;
+};
+
 // Matrix-free operator of one hex bucket (matfree.cu): elements in batches of
 // 32 in the mesh's own order, padded; built at the first solve that uses it
 struct MatFree {
@@ -145,16 +151,23 @@ struct MatFree {
   int nn = 0, nb = 0;              // nodes per element, batches
   int per_sm32 = 1, per_sm64 = 1;  // resident blocks of the element kernels
   int32_t *conn = nullptr;         // [nb][nn][32]
-  int32_t *inv = nullptr;          // [ne] colour-sorted position
+  int32_t *at = nullptr;           // [32 nb] colour-sorted position of a slot's element (padding: its complement)
   int32_t *ptr = nullptr, *inc = nullptr;  // per node: its entries of F, in fours
   float *g32 = nullptr;            // geometry at the Gauss points
-  double *g64 = nullptr;
+  double *g64 = nullptr;           // (hex20 only)
   float *lam32 = nullptr, *mu32 = nullptr;   // [nb][32]
   double *lam64 = nullptr, *mu64 = nullptr;
   float *F32 = nullptr;            // [nb][nn][32][4] element forces and a zero entry
   double *F64 = nullptr;
   float *dj32 = nullptr;           // [nnode][4] inverse diagonal (Jacobi)
   double *dj64 = nullptr;
+  // independent problems, in the order of their sizes: batches and node tiles of each
+  std::vector<int32_t> h_eptr, h_ntile;
+  int32_t *bprob = nullptr;
+  int4 *ntile = nullptr;
+  int32_t *eptr = nullptr, *nptr = nullptr;
+  double *bpart = nullptr;
+  MfProblem *S = nullptr;
   void release();
 };
 
@@ -247,6 +260,7 @@ struct Ctx {
   // independent problems in one mesh (fast_gpu_set_problems)
   int32_t nprob = 0;
   std::vector<int64_t> h_noff;    // [nprob+1] node offsets
+  std::vector<int32_t> h_order;   // problems, largest first
   int64_t *d_noff = nullptr;
   int32_t *d_order = nullptr;     // problems by size, largest first
   int32_t *d_piters = nullptr, *d_pdone = nullptr;
@@ -464,6 +478,10 @@ template <typename T>
 void mf_iterations(Ctx &c, int k, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr);
 cudaError_t mf_residual_of(Ctx &c, const double *f, const double *u, double *r, double *part, int nparts,
                            const int32_t *skip);
+// whether the independent problems are solved matrix-free, and that solve
+// (mf_prepare first); results per problem
+bool mf_batch_active(const Ctx &c);
+cudaError_t mf_solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it, double *err, int32_t *done);
 // PCG on the padded node vectors c.d_f -> c.d_u; state left in c.h_state
 cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int iter0 = 0);
 cudaError_t pcg_mixed(Ctx &c, bool warm, double tol, int maxit, int chunk);

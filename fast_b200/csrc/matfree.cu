@@ -41,12 +41,14 @@ namespace {
 
 constexpr int kT20 = 96;   // hex20: a warp per Gauss plane
 constexpr int kT8 = 128;   // hex8: 4 batches
+constexpr int kMfBatchChunk = 32;  // iterations of independent problems between two looks at their states
 
 template <typename T>
 struct MfArgs {
   int nb;                          // batches of 32 elements
   const int32_t *conn;             // [nb][nn][32] nodes (padding elements: node 0, zero geometry)
-  const T *geo;                    // hex20 [nb][9 lines][27][32], hex8 [nb][72][32]
+  const T *geo;                    // hex20 [nb][9 lines][27][32], hex8 (FP32) [nb][72][32]
+  const double *X;                 // hex8 (FP64): nodal coordinates, 3 per node
   const T *lam, *mu;               // [nb][32]
   const T *p, *z;                  // directions
   T *F;                            // [nb][nn][32][4] element forces
@@ -315,10 +317,13 @@ __global__ void __launch_bounds__(kT20, sizeof(T) == 4 ? 4 : 3) mf_hex20(MfArgs<
   if (DIR) commit_direction(A.st, done, rr, zr, err, bt);
 }
 
-// ... of the hex8 batches: a lane takes its element whole.  The geometry of a
-// warp's batch (9 or 18 KB) is copied to shared memory while the warp gathers.
-template <typename T, bool DIR>
-__global__ void __launch_bounds__(kT8) mf_hex8(MfArgs<T> A) {
+// ... of the hex8 batches in FP32: a lane takes its element whole.  The geometry
+// of a warp's batch (9 KB) is copied to shared memory while the warp gathers.
+// (Stored, not rebuilt as in FP64: differences of FP32 coordinates would lose
+// digits.)
+template <bool DIR>
+__global__ void __launch_bounds__(kT8) mf_hex8_32(MfArgs<float> A) {
+  using T = float;
   extern __shared__ __align__(16) unsigned char msm[];
   __shared__ double sred[32];
   if (A.skip && *A.skip) return;
@@ -400,6 +405,138 @@ __global__ void __launch_bounds__(kT8) mf_hex8(MfArgs<T> A) {
   if (DIR) commit_direction(A.st, done, rr, zr, err, bt);
 }
 
+// A = det J J^-1 from J (J[3 c + d] = dx_c/dxi_d); returns det J
+template <typename T>
+__device__ __forceinline__ T cofactors(const T *J, T *A) {
+  A[0] = J[4] * J[8] - J[5] * J[7];
+  A[1] = J[2] * J[7] - J[1] * J[8];
+  A[2] = J[1] * J[5] - J[2] * J[4];
+  A[3] = J[5] * J[6] - J[3] * J[8];
+  A[4] = J[0] * J[8] - J[2] * J[6];
+  A[5] = J[2] * J[3] - J[0] * J[5];
+  A[6] = J[3] * J[7] - J[4] * J[6];
+  A[7] = J[1] * J[6] - J[0] * J[7];
+  A[8] = J[0] * J[4] - J[1] * J[3];
+  return J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
+}
+
+// FP64 forces of a lane's hex8 element at x = z + beta p (DIR) or p, into
+// F[node][32][4]; returns x . K_e x.  The geometry is rebuilt from the nodes'
+// coordinates (in L1 and L2: neighbours share them): 72 stored numbers a
+// visit would be 576 of an element's 900 bytes, and the 450 extra operations
+// are cheap beside them.  The coordinates' derivatives wait in the lane's
+// column of sJ[36][kT8].  Bound by the FP64 pipe (half busy) and its latency at
+// 8 warps per SM: 248 registers hold D and R; at 168, three blocks, the spills
+// cost more than the warps give (261 against 183 us for 1.5 million elements,
+// which with loads at their point of use took 245).  An iteration at 127,500
+// nodes went from 48.9 us with stored geometry to 44.0.
+template <bool DIR>
+__device__ __forceinline__ double hex8_forces(const int32_t (&n)[8], const double *__restrict__ X, const double *p,
+                                              const double *z, double beta, double lam, double mu, double *sJ,
+                                              double *F) {
+  double D[3][3][4], R[3][3][4];
+  {
+    double x[3][8], y[3][8], v[3][8];  // every load in flight before the first use
+#pragma unroll
+    for (int a = 0; a < 8; a++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) v[c][a] = X[3 * (int64_t)n[a] + c];
+#pragma unroll
+    for (int a = 0; a < 8; a++) V4<double>::load(p + 4 * (int64_t)n[a], x[0][a], x[1][a], x[2][a]);
+    if (DIR) {
+#pragma unroll
+      for (int a = 0; a < 8; a++) V4<double>::load(z + 4 * (int64_t)n[a], y[0][a], y[1][a], y[2][a]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      mf::hex8_grads(v[c], D[c]);
+#pragma unroll
+      for (int i = 0; i < 12; i++) sJ[(12 * c + i) * kT8] = D[c][i / 4][i % 4];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (DIR) {
+#pragma unroll
+        for (int a = 0; a < 8; a++) x[c][a] = y[c][a] + beta * x[c][a];
+      }
+      mf::hex8_grads(x[c], D[c]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+#pragma unroll
+    for (int i = 0; i < 12; i++) R[c][i / 4][i % 4] = 0.0;
+#pragma unroll
+  for (int g = 0; g < 8; g++) {
+    const int gx = g & 1, gy = (g >> 1) & 1, gz = g >> 2;
+    const int id[3] = {gy + 2 * gz, gx + 2 * gz, gx + 2 * gy};
+    double H[9], P[9], A[9];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) P[3 * c + d] = sJ[(12 * c + 4 * d + id[d]) * kT8];
+    const double q = 1.0 / cofactors(P, A);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) H[3 * c + d] = D[c][d][id[d]];
+    mf::point_stress(H, A, q * lam, q * mu, P);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) R[c][d][id[d]] += P[3 * c + d];
+  }
+  double e = 0.0;  // x . G^T R = (G x) . R
+  double f[3][8];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+#pragma unroll
+    for (int i = 0; i < 12; i++) e += D[c][i / 4][i % 4] * R[c][i / 4][i % 4];
+    mf::hex8_grads_t(R[c], f[c]);
+  }
+#pragma unroll
+  for (int a = 0; a < 8; a++) V4<double>::store(F + 4 * 32 * a, f[0][a], f[1][a], f[2][a]);
+  return e;
+}
+
+// what a lane needs of its next element, loaded while it works on this one
+struct Hex8Ahead {
+  int32_t n[8];
+  double lam, mu;
+  __device__ __forceinline__ void load(const MfArgs<double> &A, int b, int lane) {
+#pragma unroll
+    for (int a = 0; a < 8; a++) n[a] = A.conn[((size_t)b * 8 + a) * 32 + lane];
+    lam = A.lam[(size_t)b * 32 + lane];
+    mu = A.mu[(size_t)b * 32 + lane];
+  }
+};
+
+template <bool DIR>
+__global__ void __launch_bounds__(kT8, 2) mf_hex8_64(MfArgs<double> A) {
+  __shared__ double sJ[36 * kT8];
+  __shared__ double sred[32];
+  if (A.skip && *A.skip) return;
+  const int tid = threadIdx.x, lane = tid & 31;
+  double pacc = 0.0, rr = 0, zr = 0, err = 0, beta = 0;
+  int done = 0;
+  if (DIR) done = next_direction<kT8>(A.st, A.part_rr, A.part_zr, A.nred, rr, zr, err, beta);
+  Hex8Ahead h;
+  int b = blockIdx.x * (kT8 / 32) + (tid >> 5);
+  if (b < A.nb) h.load(A, b, lane);
+  while (b < A.nb && !done) {
+    const Hex8Ahead g = h;
+    const int at = b;
+    b += gridDim.x * (kT8 / 32);
+    if (b < A.nb) h.load(A, b, lane);
+    pacc += hex8_forces<DIR>(g.n, A.X, A.p, A.z, beta, g.lam, g.mu, sJ + tid, A.F + 4 * ((size_t)at * (8 * 32) + lane));
+  }
+  if (A.part && !done) {
+    const double s = block_sum<kT8>(pacc, sred);
+    if (tid == 0) A.part[blockIdx.x] = s;
+  }
+  if (DIR) commit_direction(A.st, done, rr, zr, err, beta);
+}
+
 // sum of the node's element forces, supports masked
 template <typename T>
 __device__ __forceinline__ void node_force(int64_t n, const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc,
@@ -424,10 +561,44 @@ __device__ __forceinline__ void node_force(int64_t n, const int32_t *__restrict_
   if (m & 4) w2 = T(0);
 }
 
+// one node: p = z + beta p (DIR), u += alpha p, r -= alpha w, z = Dinv r; adds
+// to r.r and z.r.  dj: the inverse diagonal, 4 per node (Jacobi), or null and
+// dinv, 12 per node.
+template <typename T, bool DIR>
+__device__ __forceinline__ void node_update(int64_t n, const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc,
+                                            const T *__restrict__ F, const uint8_t *__restrict__ fix,
+                                            T *__restrict__ u, T *__restrict__ r, T *__restrict__ z,
+                                            T *__restrict__ p, const T *__restrict__ dj, const T *__restrict__ dinv,
+                                            T alpha, T beta, double &rr, double &zr) {
+  T u0, u1, u2, p0, p1, p2, r0, r1, r2, w0, w1, w2, z0, z1, z2;
+  V4<T>::load(p + 4 * n, p0, p1, p2);
+  if (DIR) V4<T>::load(z + 4 * n, z0, z1, z2);
+  V4<T>::load(u + 4 * n, u0, u1, u2);
+  V4<T>::load(r + 4 * n, r0, r1, r2);
+  node_force(n, ptr, inc, F, fix, w0, w1, w2);
+  if (DIR) {
+    p0 = z0 + beta * p0; p1 = z1 + beta * p1; p2 = z2 + beta * p2;
+    V4<T>::store(p + 4 * n, p0, p1, p2);
+  }
+  u0 = u0 + alpha * p0; u1 = u1 + alpha * p1; u2 = u2 + alpha * p2;
+  r0 = r0 + (-alpha) * w0; r1 = r1 + (-alpha) * w1; r2 = r2 + (-alpha) * w2;
+  if (dj) {
+    T d0, d1, d2;
+    V4<T>::load(dj + 4 * n, d0, d1, d2);
+    z0 = d0 * r0; z1 = d1 * r1; z2 = d2 * r2;
+  } else {
+    apply_dinv(dinv + 12 * n, r0, r1, r2, z0, z1, z2);
+  }
+  V4<T>::store(u + 4 * n, u0, u1, u2);
+  V4<T>::store(r + 4 * n, r0, r1, r2);
+  V4<T>::store(z + 4 * n, z0, z1, z2);
+  rr += (double)r0 * r0 + (double)r1 * r1 + (double)r2 * r2;
+  zr += (double)z0 * r0 + (double)z1 * r1 + (double)z2 * r2;
+}
+
 // alpha = dot0 / p.Kp (every block), p = z + beta p (DIR), u += alpha p;
 // r -= alpha w; z = Dinv r; partials r.r, z.r; the last block stores p.Kp and
-// alpha, or the breakdown state (as pcg_update_fused).  dj: the inverse
-// diagonal, 4 per node (Jacobi), or null and dinv, 12 per node.
+// alpha, or the breakdown state (as pcg_update_fused).
 template <typename T, bool DIR>
 __global__ void __launch_bounds__(kVecThreads)
 mf_update(int64_t nnode, const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc, const T *__restrict__ F,
@@ -446,33 +617,8 @@ mf_update(int64_t nnode, const int32_t *__restrict__ ptr, const int32_t *__restr
   if (!bad) {
     double rr = 0.0, zr = 0.0;
     const T alpha = (T)al;
-    for (int64_t n = blockIdx.x * (int64_t)kVecThreads + threadIdx.x; n < nnode;
-         n += (int64_t)gridDim.x * kVecThreads) {
-      T u0, u1, u2, p0, p1, p2, r0, r1, r2, w0, w1, w2, z0, z1, z2;
-      V4<T>::load(p + 4 * n, p0, p1, p2);
-      if (DIR) V4<T>::load(z + 4 * n, z0, z1, z2);
-      V4<T>::load(u + 4 * n, u0, u1, u2);
-      V4<T>::load(r + 4 * n, r0, r1, r2);
-      node_force(n, ptr, inc, F, fix, w0, w1, w2);
-      if (DIR) {
-        p0 = z0 + beta * p0; p1 = z1 + beta * p1; p2 = z2 + beta * p2;
-        V4<T>::store(p + 4 * n, p0, p1, p2);
-      }
-      u0 = u0 + alpha * p0; u1 = u1 + alpha * p1; u2 = u2 + alpha * p2;
-      r0 = r0 + (-alpha) * w0; r1 = r1 + (-alpha) * w1; r2 = r2 + (-alpha) * w2;
-      if (dj) {
-        T d0, d1, d2;
-        V4<T>::load(dj + 4 * n, d0, d1, d2);
-        z0 = d0 * r0; z1 = d1 * r1; z2 = d2 * r2;
-      } else {
-        apply_dinv(dinv + 12 * n, r0, r1, r2, z0, z1, z2);
-      }
-      V4<T>::store(u + 4 * n, u0, u1, u2);
-      V4<T>::store(r + 4 * n, r0, r1, r2);
-      V4<T>::store(z + 4 * n, z0, z1, z2);
-      rr += (double)r0 * r0 + (double)r1 * r1 + (double)r2 * r2;
-      zr += (double)z0 * r0 + (double)z1 * r1 + (double)z2 * r2;
-    }
+    for (int64_t n = blockIdx.x * (int64_t)kVecThreads + threadIdx.x; n < nnode; n += (int64_t)gridDim.x * kVecThreads)
+      node_update<T, DIR>(n, ptr, inc, F, fix, u, r, z, p, dj, dinv, alpha, beta, rr, zr);
     const double t1 = block_sum<kVecThreads>(rr, sbuf);
     if (threadIdx.x == 0) part_rr[blockIdx.x] = t1;
     const double t2 = block_sum<kVecThreads>(zr, sbuf);
@@ -505,23 +651,175 @@ mf_residual(int64_t nnode, const int32_t *__restrict__ ptr, const int32_t *__res
   if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
+// ---- independent problems, all of them an iteration at a time
+
+// Four kernels an iteration: elements (batches of every running problem, shared
+// out over resident warps), alpha, nodes (blocks of 256 of one problem), beta.
+// The chip is filled whatever the mix of sizes, and nothing streams a matrix
+// (3.4 GB an iteration for 256 cantilevers with 1.8 million nodes).  There:
+// elements 183 us on average over the solve, nodes 143 (at 5.4 TB/s), alpha and
+// beta 4.8 and 3.9; all problems 780 -> 236 ms.  (The last tile of a problem
+// forming alpha or beta behind a fence and a counter: 317 instead of 268 ms for
+// assembly and solve.)
+struct MfBatch {
+  const int32_t *bprob;  // [nb] problem of a batch
+  const int4 *ntile;     // {first node, end, problem, }
+  const int32_t *eptr;   // [nprob + 1] batches of a problem
+  const int32_t *nptr;   // ... node tiles
+  MfProblem *S;
+  double *part_pw;            // per batch
+  double *part_rr, *part_zr;  // per node tile
+};
+
+// element forces at z + beta p, p.K p per batch
+__global__ void __launch_bounds__(kT8, 2) mf_batch_elements(MfArgs<double> A, MfBatch B) {
+  __shared__ double sJ[36 * kT8];
+  const int tid = threadIdx.x, lane = tid & 31;
+  struct Next {
+    Hex8Ahead e;
+    double beta;
+    int done;
+    __device__ __forceinline__ void load(const MfArgs<double> &A, const MfBatch &B, int b, int k, int lane) {
+      e.load(A, b, lane);
+      beta = B.S[k].beta;
+      done = B.S[k].done;
+    }
+  } h;
+  const int step = gridDim.x * (kT8 / 32);
+  int b = blockIdx.x * (kT8 / 32) + (tid >> 5), k2 = 0;
+  if (b < A.nb) h.load(A, B, b, B.bprob[b], lane);
+  if (b + step < A.nb) k2 = B.bprob[b + step];
+  while (b < A.nb) {
+    const Next g = h;
+    const int at = b;
+    b += step;
+    if (b < A.nb) h.load(A, B, b, k2, lane);
+    if (b + step < A.nb) k2 = B.bprob[b + step];
+    if (g.done) continue;
+    const double e = warp_sum(hex8_forces<true>(g.e.n, A.X, A.p, A.z, g.beta, g.e.lam, g.e.mu, sJ + tid,
+                                                A.F + 4 * ((size_t)at * (8 * 32) + lane)));
+    if (lane == 0) B.part_pw[at] = e;
+  }
+}
+
+// a block per problem
+__global__ void __launch_bounds__(128) mf_batch_alpha(MfBatch B) {
+  __shared__ double sbuf[32];
+  MfProblem *S = B.S + blockIdx.x;
+  if (S->done) return;
+  double v = 0.0;
+  for (int i = B.eptr[blockIdx.x] + threadIdx.x; i < B.eptr[blockIdx.x + 1]; i += 128) v += B.part_pw[i];
+  const double pw = block_sum<128>(v, sbuf);
+  if (threadIdx.x == 0) {
+    const double al = S->dot0 / pw;
+    S->alpha = al;
+    if (!(al > 0.0) || !isfinite(pw) || !isfinite(al)) S->done = 3;
+  }
+}
+
+// p = z + beta p, u, r, z; r.r and z.r
+__global__ void __launch_bounds__(kVecThreads)
+mf_batch_update(const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc, const double *__restrict__ F,
+                const uint8_t *__restrict__ fix, double *__restrict__ u, double *__restrict__ r,
+                double *__restrict__ z, double *__restrict__ p, const double *__restrict__ dj,
+                const double *__restrict__ dinv, MfBatch B) {
+  __shared__ double sbuf[32];
+  const int4 t = B.ntile[blockIdx.x];
+  const MfProblem *S = B.S + t.z;
+  if (S->done) return;
+  const double alpha = S->alpha, beta = S->beta;
+  const int64_t n = t.x + (int)threadIdx.x;
+  double rr = 0.0, zr = 0.0;
+  if (n < t.y) node_update<double, true>(n, ptr, inc, F, fix, u, r, z, p, dj, dinv, alpha, beta, rr, zr);
+  rr = block_sum<kVecThreads>(rr, sbuf);
+  zr = block_sum<kVecThreads>(zr, sbuf);
+  if (threadIdx.x == 0) {
+    B.part_rr[blockIdx.x] = rr;
+    B.part_zr[blockIdx.x] = zr;
+  }
+}
+
+// the stopping test and beta, a block per problem
+__global__ void __launch_bounds__(128) mf_batch_beta(MfBatch B, double tol, int maxit) {
+  __shared__ double sbuf[32];
+  MfProblem *S = B.S + blockIdx.x;
+  if (S->done) return;
+  double a = 0.0, b = 0.0;
+  for (int i = B.nptr[blockIdx.x] + threadIdx.x; i < B.nptr[blockIdx.x + 1]; i += 128) {
+    a += B.part_rr[i];
+    b += B.part_zr[i];
+  }
+  const double rr = block_sum<128>(a, sbuf), zr = block_sum<128>(b, sbuf);
+  if (threadIdx.x == 0) {
+    const double err = sqrt(rr) / S->lenf;
+    S->err = err;
+    S->iter += 1;
+    S->beta = zr / S->dot0;
+    S->dot0 = zr;
+    if (err < tol) S->done = 1;
+    else if (!isfinite(err)) S->done = 3;
+    else if (S->iter >= maxit) S->done = 2;
+  }
+}
+
+// a block per problem: |f| with the reference's normaliser, r = f unless warm
+// (then r = f - K u is there), z = Dinv r, p = 0 (the first direction is z + 0 p)
+__global__ void __launch_bounds__(1024)
+mf_batch_init(const int32_t *__restrict__ order, const int64_t *__restrict__ noff,
+              const double *__restrict__ f, const double *__restrict__ dinv, double *__restrict__ u,
+              double *__restrict__ r, double *__restrict__ z, double *__restrict__ p, double tol, int warm,
+              MfProblem *__restrict__ S) {
+  __shared__ double sbuf[32];
+  __shared__ double slen;
+  const int k = order[blockIdx.x];
+  const int64_t n0 = noff[k], n1 = noff[k + 1];
+  double ff = 0.0;
+  for (int64_t n = n0 + threadIdx.x; n < n1; n += 1024) {
+    double f0, f1, f2;
+    V4<double>::load(f + 4 * n, f0, f1, f2);
+    ff += f0 * f0 + f1 * f1 + f2 * f2;
+  }
+  ff = block_sum<1024>(ff, sbuf);
+  if (threadIdx.x == 0) slen = sqrt(ff);
+  __syncthreads();
+  const double lenf = slen;
+  const bool trivial = lenf < tol;  // PCGSolver returns u = 0 at once
+  double zr = 0.0;
+  for (int64_t n = n0 + threadIdx.x; n < n1; n += 1024) {
+    double r0, r1, r2, z0, z1, z2;
+    if (trivial || !warm) V4<double>::store(u + 4 * n, 0.0, 0.0, 0.0);
+    if (trivial) continue;
+    V4<double>::load((warm ? r : f) + 4 * n, r0, r1, r2);
+    if (!warm) V4<double>::store(r + 4 * n, r0, r1, r2);
+    apply_dinv(dinv + 12 * n, r0, r1, r2, z0, z1, z2);
+    V4<double>::store(z + 4 * n, z0, z1, z2);
+    V4<double>::store(p + 4 * n, 0.0, 0.0, 0.0);
+    zr += z0 * r0 + z1 * r1 + z2 * r2;
+  }
+  zr = block_sum<1024>(zr, sbuf);
+  if (threadIdx.x == 0) S[blockIdx.x] = MfProblem{lenf > 1e11 ? 1.0 : lenf, zr, 0.0, 0.0, 0.0, 0, trivial ? 1 : 0};
+}
+
 // ---- set-up
 
-// colour-sorted incidence -> batches of 32 in the mesh's own element order
-__global__ void mf_batch_conn(int64_t ne, int64_t n32, int nn, const int32_t *__restrict__ inv,
-                              const int32_t *__restrict__ conn, int32_t *__restrict__ out) {
+// Slots: 32 per batch, at[slot] the colour-sorted position of its element, or
+// ~position for padding (an element of the batch once more, without stiffness).
+
+// colour-sorted incidence -> batches
+__global__ void mf_batch_conn(int64_t n32, int nn, const int32_t *__restrict__ at, const int32_t *__restrict__ conn,
+                              int32_t *__restrict__ out) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n32 * nn) return;
-  const int lane = (int)(t & 31);
-  const int64_t ba = t >> 5, b = ba / nn, a = ba - b * nn, e = 32 * b + lane;
-  out[t] = e < ne ? conn[(int64_t)inv[e] * nn + a] : 0;
+  const int64_t ba = t >> 5, b = ba / nn, a = ba - b * nn;
+  const int32_t i = at[32 * b + (t & 31)];
+  out[t] = conn[(int64_t)(i < 0 ? ~i : i) * nn + a];
 }
 
 // the node lists of the gathered internal force (offsets 3 (position nn + a)
 // into the colour-sorted element forces) -> entries of the batched forces, in
 // fours, padded with the zero entry
 __global__ void mf_lists(int64_t nnode, int nn, int32_t zero, const int64_t *__restrict__ gptr,
-                         const int64_t *__restrict__ ginc, const int32_t *__restrict__ perm,
+                         const int64_t *__restrict__ ginc, const int32_t *__restrict__ slot,
                          const int32_t *__restrict__ ptr, int32_t *__restrict__ inc) {
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nnode) return;
@@ -531,22 +829,23 @@ __global__ void mf_lists(int64_t nnode, int nn, int32_t zero, const int64_t *__r
     int32_t at = zero;
     if (i < i1) {
       const int64_t off = ginc[i] / 3, pos = off / nn, a = off - pos * nn;
-      const int32_t e = perm[pos];
+      const int32_t e = slot[pos];
       at = (int32_t)(((int64_t)(e >> 5) * nn + a) * 32 + (e & 31));
     }
     inc[o] = at;
   }
 }
 
-// lambda, mu per element in the mesh's own order, times `scale` (a power of two)
-__global__ void mf_material(int64_t ne, int64_t n32, double scale, const int32_t *__restrict__ inv,
-                            const double *__restrict__ E, const double *__restrict__ nu, double *__restrict__ lam,
-                            double *__restrict__ mu, float *__restrict__ lam32, float *__restrict__ mu32) {
+// lambda, mu per slot, times `scale` (a power of two)
+__global__ void mf_material(int64_t n32, double scale, const int32_t *__restrict__ at, const double *__restrict__ E,
+                            const double *__restrict__ nu, double *__restrict__ lam, double *__restrict__ mu,
+                            float *__restrict__ lam32, float *__restrict__ mu32) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= n32) return;
   double l = 0.0, m = 0.0;
-  if (e < ne) {
-    const double Ey = E[inv[e]], n = nu[inv[e]];
+  const int32_t i = at[e];
+  if (i >= 0) {
+    const double Ey = E[i], n = nu[i];
     l = scale * (Ey * n / ((1.0 + n) * (1.0 - 2.0 * n)));
     m = scale * (0.5 * Ey / (1.0 + n));
   }
@@ -558,24 +857,15 @@ __global__ void mf_material(int64_t ne, int64_t n32, double scale, const int32_t
   }
 }
 
-// A = sqrt(w det J) J^-1 from J (J[3 c + d] = dx_c/dxi_d)
+// A = sqrt(w / det J) det J J^-1 from J (det > 0: the assembly has checked it)
 __device__ __forceinline__ void point_geometry(const double *J, double w, double *A) {
-  const double c0 = J[4] * J[8] - J[5] * J[7], c1 = J[5] * J[6] - J[3] * J[8], c2 = J[3] * J[7] - J[4] * J[6];
-  const double det = J[0] * c0 + J[1] * c1 + J[2] * c2;
-  const double s = sqrt(w / det);  // (det > 0: the assembly has checked it)
-  A[0] = s * c0;
-  A[1] = s * (J[2] * J[7] - J[1] * J[8]);
-  A[2] = s * (J[1] * J[5] - J[2] * J[4]);
-  A[3] = s * c1;
-  A[4] = s * (J[0] * J[8] - J[2] * J[6]);
-  A[5] = s * (J[2] * J[3] - J[0] * J[5]);
-  A[6] = s * c2;
-  A[7] = s * (J[1] * J[6] - J[0] * J[7]);
-  A[8] = s * (J[0] * J[4] - J[1] * J[3]);
+  const double s = sqrt(w / cofactors(J, A));
+#pragma unroll
+  for (int q = 0; q < 9; q++) A[q] *= s;
 }
 
 constexpr int kG20 = 288;  // a warp per Gauss line
-__global__ void __launch_bounds__(kG20) mf_geometry20(int64_t ne, int nb, const int32_t *__restrict__ conn,
+__global__ void __launch_bounds__(kG20) mf_geometry20(int nb, const int32_t *__restrict__ conn,
                                                       const double *__restrict__ X, double *__restrict__ g64,
                                                       float *__restrict__ g32) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = w / 3, j = w - 3 * k;
@@ -591,7 +881,6 @@ __global__ void __launch_bounds__(kG20) mf_geometry20(int64_t ne, int nb, const 
       for (int q = 0; q < 8; q++) L[c][q] *= 1.0 / mf::kScale20;
     }
     mf::line_gradients(L, H);
-    const bool real = 32 * (int64_t)b + lane < ne;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
       const double wt = (i == 1 ? 8.0 : 5.0) * (j == 1 ? 8.0 : 5.0) * (k == 1 ? 8.0 : 5.0) / 729.0;
@@ -600,17 +889,15 @@ __global__ void __launch_bounds__(kG20) mf_geometry20(int64_t ne, int nb, const 
 #pragma unroll
       for (int q = 0; q < 9; q++) {
         const size_t at = (((size_t)b * 9 + w) * 27 + 9 * i + q) * 32 + lane;
-        const double v = real ? A[q] : 0.0;
-        g64[at] = v;
-        if (g32) g32[at] = (float)v;
+        g64[at] = A[q];
+        if (g32) g32[at] = (float)A[q];
       }
     }
   }
 }
 
-__global__ void __launch_bounds__(kT8) mf_geometry8(int64_t ne, int nb, const int32_t *__restrict__ conn,
-                                                    const double *__restrict__ X, double *__restrict__ g64,
-                                                    float *__restrict__ g32) {
+__global__ void __launch_bounds__(kT8) mf_geometry8(int nb, const int32_t *__restrict__ conn,
+                                                    const double *__restrict__ X, float *__restrict__ g32) {
   const int lane = threadIdx.x & 31;
   for (int b = blockIdx.x * (kT8 / 32) + (threadIdx.x >> 5); b < nb; b += gridDim.x * (kT8 / 32)) {
     double D[3][3][4];
@@ -620,7 +907,6 @@ __global__ void __launch_bounds__(kT8) mf_geometry8(int64_t ne, int nb, const in
       for (int a = 0; a < 8; a++) f[a] = X[3 * (int64_t)conn[((size_t)b * 8 + a) * 32 + lane] + c];
       mf::hex8_grads(f, D[c]);
     }
-    const bool real = 32 * (int64_t)b + lane < ne;
 #pragma unroll
     for (int g = 0; g < 8; g++) {
       const int gx = g & 1, gy = (g >> 1) & 1, gz = g >> 2;
@@ -634,10 +920,7 @@ __global__ void __launch_bounds__(kT8) mf_geometry8(int64_t ne, int nb, const in
       point_geometry(J, 1.0, A);
 #pragma unroll
       for (int q = 0; q < 9; q++) {
-        const size_t at = ((size_t)b * 72 + 9 * g + q) * 32 + lane;
-        const double v = real ? A[q] : 0.0;
-        g64[at] = v;
-        if (g32) g32[at] = (float)v;
+        g32[((size_t)b * 72 + 9 * g + q) * 32 + lane] = (float)A[q];
       }
     }
   }
@@ -651,7 +934,7 @@ __global__ void mf_diag(int64_t nnode, const T *__restrict__ dinv, T *__restrict
   V4<T>::store(dj + 4 * n, dinv[12 * n], dinv[12 * n + 5], dinv[12 * n + 10]);
 }
 
-template <typename T> constexpr size_t kSmem8 = (kT8 / 32) * 72 * 32 * sizeof(T);
+constexpr size_t kSmem8 = (kT8 / 32) * 72 * 32 * sizeof(float);  // mf_hex8_32
 template <typename T> constexpr size_t kSmem20 = (3 * 20 + 3 * (sizeof(T) == 4 ? 81 : 72)) * 32 * sizeof(T) + 20 * 32 * sizeof(int32_t);
 
 template <typename T>
@@ -672,19 +955,21 @@ template <typename T, bool DIR>
 void mf_elements(Ctx &c, const T *p, const T *z, const int32_t *skip, double *part, const double *part_rr,
                  const double *part_zr, int nred) {
   const MatFree &M = c.mf;
-  const MfArgs<T> a{M.nb, M.conn, either<T>(M.g32, M.g64), either<T>(M.lam32, M.lam64), either<T>(M.mu32, M.mu64), p, z,
+  const MfArgs<T> a{M.nb, M.conn, either<T>(M.g32, M.g64), c.d_X, either<T>(M.lam32, M.lam64), either<T>(M.mu32, M.mu64), p, z,
                     either<T>(M.F32, M.F64), c.d_state, skip, part, part_rr, part_zr, nred};
   const int G = mf_grid<T>(c);
   if (M.nn == 20) mf_hex20<T, DIR><<<G, kT20, kSmem20<T>, c.stream>>>(a);
-  else mf_hex8<T, DIR><<<G, kT8, kSmem8<T>, c.stream>>>(a);
+  else if constexpr (sizeof(T) == 4) mf_hex8_32<DIR><<<G, kT8, kSmem8, c.stream>>>(a);
+  else mf_hex8_64<DIR><<<G, kT8, 0, c.stream>>>(a);
   c.launches++;
 }
 
 }  // namespace
 
 void MatFree::release() {
-  for (void *p : {(void *)conn, (void *)inv, (void *)ptr, (void *)inc, (void *)g32, (void *)g64, (void *)lam32,
-                  (void *)mu32, (void *)lam64, (void *)mu64, (void *)F32, (void *)F64, (void *)dj32, (void *)dj64})
+  for (void *p : {(void *)conn, (void *)at, (void *)ptr, (void *)inc, (void *)g32, (void *)g64, (void *)lam32,
+                  (void *)mu32, (void *)lam64, (void *)mu64, (void *)F32, (void *)F64, (void *)dj32, (void *)dj64,
+                  (void *)bprob, (void *)ntile, (void *)eptr, (void *)nptr, (void *)bpart, (void *)S})
     if (p) cudaFree(p);
   *this = MatFree{};
 }
@@ -697,30 +982,96 @@ void MatFree::release() {
 //   hex20  19,623 nodes FP32 11.9 / 16.7  FP64 16.3 / 18.8
 //          35,116            17.2 / 17.3       43.9 / 21.0
 //          54,398            32.4 / 19.9       85.7 / 26.1
-//   hex8   29,791            11.0 / 15.4       15.1 / 19.7
-//          64,000            17.3 / 18.4       40.6 / 26.7
-//         127,500            47.4 / 22.1       71.2 / 48.9
-bool mf_active(const Ctx &c) {
+//   hex8   29,791            10.9 / 14.8       15.0 / 18.6
+//          64,000            17.1 / 17.5       40.9 / 25.9
+//         127,500            47.0 / 22.9       70.6 / 44.0
+static bool mf_possible(const Ctx &c) {
   if (!c.K_pure || c.mf_off || c.has_ties() || c.buckets.size() != 1 || !c.force_gather) return false;
   const Bucket &B = c.buckets[0];
   if (B.tl || !((B.type == FAST_ELEM_HEX8 && B.ng == 8) || (B.type == FAST_ELEM_HEX20 && B.ng == 27))) return false;
-  const int64_t least = c.mf_min_nodes >= 0 ? c.mf_min_nodes
-                        : B.nn == 20        ? (c.mf_fp32 ? 36000 : 22000)
-                                            : (c.mf_fp32 ? 66000 : 42000);
-  return c.nnode >= least && B.ne * B.nn < (int64_t)1 << 30;
+  return (B.ne + 31 * std::max(1, (int)c.nprob)) * B.nn < (int64_t)1 << 30;
+}
+bool mf_active(const Ctx &c) {
+  if (!mf_possible(c)) return false;
+  const int64_t least = c.mf_min_nodes >= 0        ? c.mf_min_nodes
+                        : c.buckets[0].nn == 20    ? (c.mf_fp32 ? 36000 : 22000)
+                                                   : (c.mf_fp32 ? 66000 : 42000);
+  return c.nnode >= least;
+}
+// Independent hex8 problems: all of them an iteration at a time, or a cluster of
+// two blocks for each on the assembled matrix (pcg_batch)?  Fitted to solves of
+// 1 to 1,000 cantilevers of 45 to 18,081 nodes each: an iteration of pcg_batch
+// takes 6.5 us and 0.036 us per node of its problem, 148 clusters run at once
+// and the largest problem may be what is waited for; a lockstep iteration takes
+// 24 us (four kernels) and 0.15 ns per node of all problems.  Measured, ms
+// (pcg_batch / lockstep): 8 problems of 112..637 nodes 5.6 / 5.1, 16 of 112..396
+// 3.1 / 4.3, 64 of 45..112 1.1 / 2.9, 128 of 112..637 6.5 / 6.3, 256 of 225..1,377
+// 26 / 16, 1,000 of 45 3.8 / 3.3, 8 of 1,900..18,081 501 / 23, 256 of
+// 637..18,081 780 / 236.
+bool mf_batch_active(const Ctx &c) {
+  if (c.nprob <= 0 || !mf_possible(c) || c.buckets[0].nn != 8) return false;
+  if (c.mf_min_nodes >= 0) return c.nnode >= c.mf_min_nodes;
+  double sum = 0.0, most = 0.0;
+  for (int k = 0; k < c.nprob; k++) {
+    const double t = 6.5 + 0.036 * (double)(c.h_noff[k + 1] - c.h_noff[k]);
+    sum += t;
+    most = std::max(most, t);
+  }
+  return 24.0 + 0.15e-3 * (double)c.nnode < std::max(most, sum / c.sm_count);
+}
+
+// The batches: elements in the mesh's own order, 32 at a time; of a context with
+// independent problems (fast_gpu_set_problems) problem by problem, the largest
+// first, each from a batch of its own.  at[slot]: as in mf_batch_conn;
+// slot[colour-sorted position].
+static void mf_slots(Ctx &c, std::vector<int32_t> &at, std::vector<int32_t> &slot) {
+  MatFree &M = c.mf;
+  const Bucket &B = c.buckets[0];
+  slot.resize(B.ne);
+  auto put = [&](int32_t pos) {
+    slot[pos] = (int32_t)at.size();
+    at.push_back(pos);
+  };
+  auto pad = [&] {
+    const int32_t last = at.empty() ? 0 : at.back();
+    while (at.size() % 32) at.push_back(~last);
+  };
+  M.h_eptr.clear();
+  if (c.nprob <= 0) {
+    for (int64_t e = 0; e < B.ne; e++) put(B.inv[e]);
+    pad();
+    return;
+  }
+  std::vector<int32_t> rank(c.nprob);
+  for (int k = 0; k < c.nprob; k++) rank[c.h_order[k]] = k;
+  std::vector<std::vector<int32_t>> of(c.nprob);
+  for (int64_t e = 0; e < B.ne; e++) {
+    const int64_t n = B.h_conn[(int64_t)B.inv[e] * B.nn];
+    const auto up = std::upper_bound(c.h_noff.begin(), c.h_noff.end(), n);
+    of[rank[up - c.h_noff.begin() - 1]].push_back(B.inv[e]);
+  }
+  for (int k = 0; k < c.nprob; k++) {
+    M.h_eptr.push_back((int32_t)(at.size() / 32));
+    for (int32_t pos : of[k]) put(pos);
+    pad();
+  }
+  M.h_eptr.push_back((int32_t)(at.size() / 32));
 }
 
 // the batched copies of mesh, geometry and material, whichever are stale
 cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
   MatFree &M = c.mf;
   const Bucket &B = c.buckets[0];
-  const int64_t ne = B.ne, nn = B.nn, n32 = (ne + 31) / 32 * 32;
+  const int64_t ne = B.ne, nn = B.nn;
   const size_t ng9 = (size_t)9 * B.ng;
   cudaError_t e = cudaSuccess;
   auto alloc = [&](auto **p, size_t n) {
     if (e == cudaSuccess && !*p) e = cudaMalloc((void **)p, sizeof(**p) * n);
   };
   if (!M.built) {
+    std::vector<int32_t> at, slot;
+    mf_slots(c, at, slot);
+    const int64_t n32 = (int64_t)at.size();
     M.nn = (int)nn;
     M.nb = (int)(n32 / 32);
     std::vector<int64_t> gptr(c.nnode + 1);
@@ -730,34 +1081,34 @@ cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
         (e = cudaStreamSynchronize(c.stream)) != cudaSuccess)
       return e;
     for (int64_t n = 0; n < c.nnode; n++) ptr[n + 1] = ptr[n] + (int32_t)((gptr[n + 1] - gptr[n] + 3) / 4);
-    int32_t *perm = nullptr;
+    int32_t *d_slot = nullptr;
     alloc(&M.conn, n32 * nn);
-    alloc(&M.inv, ne);
+    alloc(&M.at, n32);
     alloc(&M.ptr, c.nnode + 1);
     alloc(&M.inc, 4 * (size_t)ptr[c.nnode]);
     alloc(&M.lam64, n32);
     alloc(&M.mu64, n32);
-    alloc(&M.g64, n32 * ng9);
+    if (nn == 20) alloc(&M.g64, n32 * ng9);
     alloc(&M.F64, n32 * nn * 4 + 4);  // one zero entry behind the last
     if (e == cudaSuccess) e = cudaMemsetAsync(M.F64 + 4 * n32 * nn, 0, sizeof(double) * 4, c.stream);
     alloc(&M.dj64, 4 * c.nnode);
-    alloc(&perm, ne);
+    alloc(&d_slot, ne);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(M.inv, B.inv.data(), sizeof(int32_t) * ne, cudaMemcpyHostToDevice, c.stream);
+      e = cudaMemcpyAsync(M.at, at.data(), sizeof(int32_t) * n32, cudaMemcpyHostToDevice, c.stream);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(perm, B.perm.data(), sizeof(int32_t) * ne, cudaMemcpyHostToDevice, c.stream);
+      e = cudaMemcpyAsync(d_slot, slot.data(), sizeof(int32_t) * ne, cudaMemcpyHostToDevice, c.stream);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(M.ptr, ptr.data(), sizeof(int32_t) * ptr.size(), cudaMemcpyHostToDevice, c.stream);
     if (e == cudaSuccess) {
       const int64_t t1 = n32 * nn;
-      mf_batch_conn<<<(unsigned)((t1 + 255) / 256), 256, 0, c.stream>>>(ne, n32, (int)nn, M.inv, B.d_conn, M.conn);
+      mf_batch_conn<<<(unsigned)((t1 + 255) / 256), 256, 0, c.stream>>>(n32, (int)nn, M.at, B.d_conn, M.conn);
       mf_lists<<<(unsigned)((c.nnode + 255) / 256), 256, 0, c.stream>>>(c.nnode, (int)nn, (int32_t)t1, c.d_gptr,
-                                                                        c.d_ginc, perm, M.ptr, M.inc);
+                                                                        c.d_ginc, d_slot, M.ptr, M.inc);
       c.launches += 2;
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
-    if (perm) cudaFree(perm);
+    if (d_slot) cudaFree(d_slot);
     if (e != cudaSuccess) return e;
     int a = 0, b = 0;
     auto sized = [&](auto kern, int threads, size_t smem, int *n) {
@@ -770,16 +1121,17 @@ cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
       sized(mf_hex20<double, true>, kT20, kSmem20<double>, &a);
       sized(mf_hex20<float, true>, kT20, kSmem20<float>, &b);
     } else {
-      sized(mf_hex8<double, false>, kT8, kSmem8<double>, &a);
-      sized(mf_hex8<float, false>, kT8, kSmem8<float>, &b);
-      sized(mf_hex8<double, true>, kT8, kSmem8<double>, &a);
-      sized(mf_hex8<float, true>, kT8, kSmem8<float>, &b);
+      sized(mf_hex8_64<false>, kT8, 0, &a);
+      sized(mf_hex8_32<false>, kT8, kSmem8, &b);
+      sized(mf_hex8_64<true>, kT8, 0, &a);
+      sized(mf_hex8_32<true>, kT8, kSmem8, &b);
     }
     if (e != cudaSuccess) return e;
     M.per_sm64 = std::max(1, a);
     M.per_sm32 = std::max(1, b);
     M.built = true;
   }
+  const int64_t n32 = 32 * (int64_t)M.nb;
   if (fp32) {
     if (!M.g32) M.geo_ok = M.mat_ok = false;
     alloc(&M.g32, n32 * ng9);
@@ -791,17 +1143,17 @@ cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
     if (e == cudaSuccess && fresh) e = cudaMemsetAsync(M.F32 + 4 * n32 * nn, 0, sizeof(float) * 4, c.stream);
     if (e != cudaSuccess) return e;
   }
-  if (!M.geo_ok) {
+  if (!M.geo_ok && (nn == 20 || M.g32)) {
     const int G = std::min(2 * M.nb, 8 * c.sm_count);
-    if (nn == 20) mf_geometry20<<<G, kG20, 0, c.stream>>>(ne, M.nb, M.conn, c.d_X, M.g64, M.g32);
-    else mf_geometry8<<<G, kT8, 0, c.stream>>>(ne, M.nb, M.conn, c.d_X, M.g64, M.g32);
+    if (nn == 20) mf_geometry20<<<G, kG20, 0, c.stream>>>(M.nb, M.conn, c.d_X, M.g64, M.g32);
+    else mf_geometry8<<<G, kT8, 0, c.stream>>>(M.nb, M.conn, c.d_X, M.g32);
     c.launches++;
     M.geo_ok = true;
   }
   if (!M.mat_ok) {
     const double scale = nn == 20 ? 1.0 / (mf::kScale20 * mf::kScale20) : 1.0;
-    mf_material<<<(unsigned)((n32 + 255) / 256), 256, 0, c.stream>>>(ne, n32, scale, M.inv, B.d_E, B.d_nu, M.lam64,
-                                                                     M.mu64, M.lam32, M.mu32);
+    mf_material<<<(unsigned)((n32 + 255) / 256), 256, 0, c.stream>>>(n32, scale, M.at, B.d_E, B.d_nu, M.lam64, M.mu64,
+                                                                     M.lam32, M.mu32);
     c.launches++;
     M.mat_ok = true;
   }
@@ -851,6 +1203,72 @@ cudaError_t mf_residual_of(Ctx &c, const double *f, const double *u, double *r, 
   mf_residual<<<nparts, kVecThreads, 0, c.stream>>>(c.nnode, M.ptr, M.inc, M.F64, c.d_fix, f, r, part, skip);
   c.launches++;
   return cudaGetLastError();
+}
+
+// Per-problem PCG of every problem, as launch_pcg_batch.  The problems lie
+// largest first, so the launches shrink from the end as the small ones, which
+// need fewer iterations, are done.
+cudaError_t mf_solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it, double *err, int32_t *done) {
+  MatFree &M = c.mf;
+  cudaError_t e;
+  const int np = c.nprob;
+  if (!M.S) {
+    std::vector<int32_t> bp(M.nb);
+    std::vector<int4> nt;
+    M.h_ntile.assign(1, 0);
+    for (int k = 0; k < np; k++) {
+      const int64_t n0 = c.h_noff[c.h_order[k]], n1 = c.h_noff[c.h_order[k] + 1];
+      for (int b = M.h_eptr[k]; b < M.h_eptr[k + 1]; b++) bp[b] = k;
+      for (int64_t n = n0; n < n1; n += kVecThreads)
+        nt.push_back(make_int4((int)n, (int)std::min(n + kVecThreads, n1), k, 0));
+      M.h_ntile.push_back((int32_t)nt.size());
+    }
+    e = cudaSuccess;
+    auto up = [&](auto **p, const auto &v) {
+      if (e == cudaSuccess && !*p) e = cudaMalloc((void **)p, sizeof(v[0]) * std::max<size_t>(1, v.size()));
+      if (e == cudaSuccess) e = cudaMemcpy(*p, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+    };
+    up(&M.bprob, bp);
+    up(&M.ntile, nt);
+    up(&M.eptr, M.h_eptr);
+    up(&M.nptr, M.h_ntile);
+    if (e == cudaSuccess && !M.bpart) e = cudaMalloc((void **)&M.bpart, sizeof(double) * (M.nb + 2 * nt.size() + 1));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&M.S, sizeof(MfProblem) * np);
+    if (e != cudaSuccess) return e;
+  }
+  if (warm && (e = mf_residual_of(c, c.d_f, c.d_u, c.d_r, c.d_partials, kRedBlocks, nullptr)) != cudaSuccess) return e;
+  mf_batch_init<<<np, 1024, 0, c.stream>>>(c.d_order, c.d_noff, c.d_f, c.d_dinv, c.d_u, c.d_r, c.d_z, c.d_p, tol,
+                                           warm ? 1 : 0, M.S);
+  c.launches++;
+  MfArgs<double> a{M.nb, M.conn, M.g64, c.d_X, M.lam64, M.mu64, c.d_p, c.d_z, M.F64, nullptr, nullptr, nullptr, nullptr,
+                   nullptr, 0};
+  const MfBatch b{M.bprob, M.ntile, M.eptr, M.nptr, M.S, M.bpart, M.bpart + M.nb, M.bpart + M.nb + M.h_ntile[np]};
+  std::vector<MfProblem> S(np);
+  int live = np;  // problems [0, live) of the order may still run
+  for (int chunk = 0;; chunk = std::min(chunk ? 2 * chunk : 8, kMfBatchChunk)) {
+    a.nb = M.h_eptr[live];
+    const int G = std::max(1, std::min(M.per_sm64 * c.sm_count, (a.nb + kT8 / 32 - 1) / (kT8 / 32)));
+    for (int i = 0; i < chunk; i++) {
+      mf_batch_elements<<<G, kT8, 0, c.stream>>>(a, b);
+      mf_batch_alpha<<<live, 128, 0, c.stream>>>(b);
+      mf_batch_update<<<M.h_ntile[live], kVecThreads, 0, c.stream>>>(
+          M.ptr, M.inc, M.F64, c.d_fix, c.d_u, c.d_r, c.d_z, c.d_p, M.jacobi ? M.dj64 : nullptr, c.d_dinv, b);
+      mf_batch_beta<<<live, 128, 0, c.stream>>>(b, tol, maxit);
+      c.launches += 4;
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess ||
+        (e = cudaMemcpyAsync(S.data(), M.S, sizeof(MfProblem) * np, cudaMemcpyDeviceToHost, c.stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(c.stream)) != cudaSuccess)
+      return e;
+    while (live > 0 && S[live - 1].done) live--;
+    if (live == 0) break;
+  }
+  for (int k = 0; k < np; k++) {
+    it[c.h_order[k]] = S[k].iter;
+    err[c.h_order[k]] = S[k].err;
+    done[c.h_order[k]] = S[k].done;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace fastgpu

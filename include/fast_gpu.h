@@ -559,7 +559,7 @@ int fast_gpu_newmark(fast_gpu_ctx *ctx, const double *q, const fast_gpu_newmark_
  * problems: checked).  Assembly then covers all problems in one pass, and
  * fast_gpu_solve_batch solves every problem to its own PCGSolver stopping test
  * (mlib/sysmat.cpp:1061-1125: |r_k|/|f_k| < tol, |f_k| > 1e11 replaced by 1,
- * u_k = 0 when |f_k| < tol) in one launch, one CTA per problem. */
+ * u_k = 0 when |f_k| < tol) all problems at once. */
 typedef struct {
   int32_t converged;
   int32_t iterations;
