@@ -66,6 +66,7 @@ void free_mesh(Ctx &c) {
   dfree(c.d_K); dfree(c.d_M); dfree(c.d_Ks); dfree(c.d_Ms); dfree(c.d_Ks32);
   dfree(c.d_u); dfree(c.d_r); dfree(c.d_z); dfree(c.d_p); dfree(c.d_w); dfree(c.d_f); dfree(c.d_dinv);
   dfree(c.d_p2); dfree(c.s_p2);
+  dfree(c.d_mpairs);
   dfree(c.d_ubest);
   dfree(c.s_x); dfree(c.s_r); dfree(c.s_z); dfree(c.s_p); dfree(c.s_w); dfree(c.s_dinv);
   dfree(c.d_eq_tmp);
@@ -711,9 +712,13 @@ int fast_gpu_assemble(fast_gpu_ctx *c, int32_t what) {
   double *T = target_of(*c, what);
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(int32_t), c->stream));
   if (what == FAST_ASM_STIFFNESS) c->begin_span(2);
-  // (with first-touch flags every block is stored by its first writer)
-  if (!(what == FAST_ASM_STIFFNESS && c->use_first_touch())) CK(launch_zero_matrix(*c, T, what == FAST_ASM_STIFFNESS));
-  CK(launch_assemble(*c, what, T));
+  cudaError_t rows = cudaErrorNotSupported;
+  if (what == FAST_ASM_MASS && (rows = launch_mass_rows(*c, T)) != cudaErrorNotSupported) CK(rows);
+  if (rows == cudaErrorNotSupported) {
+    // (with first-touch flags every block is stored by its first writer)
+    if (!(what == FAST_ASM_STIFFNESS && c->use_first_touch())) CK(launch_zero_matrix(*c, T, what == FAST_ASM_STIFFNESS));
+    CK(launch_assemble(*c, what, T));
+  }
   if (what == FAST_ASM_STIFFNESS) CK(launch_tl(*c, T, nullptr, true, false));
   if (what == FAST_ASM_STIFFNESS) c->end_span();
   CK(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
@@ -790,9 +795,13 @@ int fast_gpu_mult_vect(fast_gpu_ctx *c, int32_t what, const double *x, double *y
   CK(cudaStreamSynchronize(c->stream));
   std::memcpy(c->h_eq_tmp, x, nb);
   CK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp, nb, cudaMemcpyHostToDevice, c->stream));
-  CK(ensure_soa(*c, what, false));
   CK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_z));
-  CK(launch_spmv(*c, what == FAST_ASM_MASS ? c->d_Ms : c->d_Ks, c->d_z, c->d_w));
+  // the solve layout where it is there: a product takes 112 us on it and 127 on
+  // the blocks (32,760 hex20 elements), but making it 240
+  if (what == FAST_ASM_MASS ? c->Ms_ok : c->Ks_ok)
+    CK(launch_spmv(*c, what == FAST_ASM_MASS ? c->d_Ms : c->d_Ks, c->d_z, c->d_w));
+  else
+    CK(launch_spmv_blocks(*c, T, c->d_z, c->d_w));
   CK(launch_node_to_eq(*c, c->d_w, c->d_eq_tmp));
   CK(cudaMemcpyAsync(c->h_eq_tmp, c->d_eq_tmp, nb, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

@@ -205,6 +205,7 @@ struct Ctx {
   // node-block (3x3) CSR pattern, full (both triangles)
   int64_t nnzb = 0;
   std::vector<int32_t> h_rowptr, h_col, h_diag;
+  double *d_mpairs = nullptr;     // [ne][nn][nn] mass per node pair (mass_rows.cu)
   int32_t *d_rowptr = nullptr, *d_col = nullptr, *d_diag = nullptr;
   // solve layout: each block-row padded to a multiple of 4 blocks, so its
   // structure-of-arrays segments start on 16-byte boundaries (vector loads)
@@ -423,6 +424,9 @@ cudaError_t launch_tie_prolong(Ctx &c, double *u);   // u[slave] = sum w u[maste
 cudaError_t launch_element_matrices(Ctx &c, int what, int bucket, int64_t first_sorted, int64_t count,
                                     double *d_out);
 
+// mass_rows.cu: every block of M stored (no zero fill); cudaErrorNotSupported
+// where launch_assemble has to add it
+cudaError_t launch_mass_rows(Ctx &c, double *M);
 // geom.cu: G += sign * geometric stiffness at c.d_disp (small-strain hex
 // buckets, colour by colour; fixed rows and columns untouched)
 cudaError_t launch_geom_stiffness(Ctx &c, double *G, double sign);
@@ -507,6 +511,8 @@ cudaError_t launch_pcg_batch(Ctx &c, int nprob, const int32_t *d_order, const in
                              bool warm, int32_t *d_iters, double *d_errs, int32_t *d_done);
 cudaError_t launch_residual(Ctx &c, const double *Ks, const double *f, const double *u, double *r,
                             double *rr_out_dev);
+// y = K x from the blocks as assembled
+cudaError_t launch_spmv_blocks(Ctx &c, const double *K, const double *x, double *y);
 cudaError_t launch_spmv(Ctx &c, const double *Ks, const double *x, double *y);
 cudaError_t launch_spmv32(Ctx &c, const float *Ks, const float *x, float *y);
 cudaError_t launch_eq_to_node(Ctx &c, const double *eqv, double *nodev);

@@ -977,6 +977,48 @@ cudaError_t launch_matfree_residual(Ctx &c, const double *f, const double *u, do
   return cudaGetLastError();
 }
 
+// y = K x from the 3x3 blocks as assembled, row-major, for a product or two of a
+// matrix that no solve has asked a layout for.  A warp per block-row; 27 lanes
+// take three whole blocks (216 bytes) at a time, each lane one entry of a
+// block, so loads are whole lines and a lane's row and column never change.
+// 563 MB in 127 us, where the solve layout's product takes 112 and making that
+// layout 240.  (Eight trips of three blocks in flight and a grid of eight blocks
+// per SM, of which five fit, took 158; six blocks per SM, with spills, 224.)
+__global__ void __launch_bounds__(kSpmvThreads, 5)
+spmv_blocks(int64_t nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
+            const double *__restrict__ K, const double *__restrict__ x, double *__restrict__ y) {
+  const int lane = threadIdx.x & 31, kb = lane / 9, k = lane - 9 * kb, j = k % 3;
+  constexpr int U = 7;  // 21 blocks in flight: hex20 rows of 51, 57 and 81, hex8 ones of 27
+  for (int64_t n = (blockIdx.x * (int64_t)kSpmvThreads + threadIdx.x) >> 5; n < nrows;
+       n += ((int64_t)gridDim.x * kSpmvThreads) >> 5) {
+    const int32_t b0 = rowptr[n], b1 = rowptr[n + 1];
+    double s = 0.0;
+    for (int32_t b = b0; b < b1; b += 3 * U) {
+      double v[U], xv[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int32_t at = b + 3 * u + kb;
+        const bool in = kb < 3 && at < b1;
+        v[u] = in ? K[9 * (int64_t)at + k] : 0.0;
+        xv[u] = in ? x[4 * (int64_t)col[at] + j] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) s += v[u] * xv[u];
+    }
+    // lanes 9 kb + 3 i + j -> row i
+    s += __shfl_down_sync(0xffffffffu, s, 9) + __shfl_down_sync(0xffffffffu, s, 18);
+    s += __shfl_down_sync(0xffffffffu, s, 1) + __shfl_down_sync(0xffffffffu, s, 2);
+    const double s1 = __shfl_down_sync(0xffffffffu, s, 3), s2 = __shfl_down_sync(0xffffffffu, s, 6);
+    if (lane == 0) V4<double>::store(y + 4 * n, s, s1, s2);
+  }
+}
+
+cudaError_t launch_spmv_blocks(Ctx &c, const double *K, const double *x, double *y) {
+  spmv_blocks<<<5 * c.sm_count, kSpmvThreads, 0, c.stream>>>(c.nnode, c.d_rowptr, c.d_col, K, x, y);
+  c.launches++;
+  return cudaGetLastError();
+}
+
 cudaError_t launch_spmv(Ctx &c, const double *Ks, const double *x, double *y) {
   spmv64_go<0>(c, spmv_grid(c), c.nnode, Ks, x, nullptr, y, nullptr, nullptr);
   c.launches++;
