@@ -46,7 +46,7 @@ void free_mesh(Ctx &c) {
   c.K_pure = false;
   for (Bucket &B : c.buckets) {
     dfree(B.d_conn); dfree(B.d_E); dfree(B.d_nu); dfree(B.d_rho); dfree(B.d_slot); dfree(B.d_first);
-    dfree(B.d_dN); dfree(B.d_N); dfree(B.d_w);
+    dfree(B.d_dN); dfree(B.d_dNt); dfree(B.d_N); dfree(B.d_w);
     dfree(B.d_span); dfree(B.d_bas); dfree(B.d_wt);
     dfree(B.d_tr); dfree(B.d_nptr); dfree(B.d_nent);
   }
@@ -507,6 +507,13 @@ int fast_gpu_upload_mesh(fast_gpu_ctx *c, const fast_gpu_mesh *m) {
     CK(cudaMemcpy(B.d_N, N.data(), sizeof(double) * N.size(), cudaMemcpyHostToDevice));
     CK(dalloc(&B.d_dN, dN.size()));
     CK(cudaMemcpy(B.d_dN, dN.data(), sizeof(double) * dN.size(), cudaMemcpyHostToDevice));
+    if (B.type == FAST_ELEM_HEX20) {
+      std::vector<double> t(dN.size());
+      for (int g = 0; g < B.ng; g++)
+        for (int i = 0; i < 3 * B.nn; i++) t[(size_t)i * B.ng + g] = dN[(size_t)g * 3 * B.nn + i];
+      CK(dalloc(&B.d_dNt, t.size()));
+      CK(cudaMemcpy(B.d_dNt, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
+    }
     CK(dalloc(&B.d_w, w.size()));
     CK(cudaMemcpy(B.d_w, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice));
   }

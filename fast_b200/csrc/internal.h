@@ -67,6 +67,7 @@ struct Bucket {
   double *d_E = nullptr, *d_nu = nullptr, *d_rho = nullptr;
   int32_t *d_slot = nullptr;       // [ne][nn][nn] block index of node pair (a, b)
   double *d_dN = nullptr;          // [ng][nn][3] natural derivatives at the Gauss points
+  double *d_dNt = nullptr;         // [nn][3][ng] the same, Gauss point innermost (hex20)
   double *d_N = nullptr;           // [ng][nn] shape functions
   double *d_w = nullptr;           // [ng] Gauss weights
   int64_t ne_regular = 0;          // colour-scheduled elements; the tied ones follow in perm order
@@ -398,6 +399,8 @@ cudaError_t launch_assemble(Ctx &c, int what, double *target);
 // elem_warp.cu: FP64 hex stiffness with one warp per element (one colour)
 struct ElemArgs;
 bool warp_supported(const Bucket &B);
+// elem_mma.cu: FP64 hex20 stiffness into K on the FP64 matrix instruction (one colour)
+cudaError_t launch_mma_elements(Ctx &c, const Bucket &B, ElemArgs a, int64_t count);
 cudaError_t launch_warp_elements(Ctx &c, const Bucket &B, ElemArgs a, int64_t count);
 // the small-strain stiffness of one bucket, every colour (no tied elements)
 cudaError_t launch_assemble_bucket(Ctx &c, size_t b, double *target);
