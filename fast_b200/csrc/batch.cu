@@ -108,11 +108,14 @@ extern "C" int fast_gpu_solve_batch(fast_gpu_ctx *c, const double *f, double *u,
   if (mf) BCK(mf_prepare(*c, false, opts.precond));
   else BCK(solve_layout(*c, FAST_ASM_STIFFNESS, false));
   const size_t nb = sizeof(double) * c->neq;
-  BCK(cudaMemcpyAsync(c->d_eq_tmp, f, nb, cudaMemcpyHostToDevice, c->stream));
+  BCK(cudaStreamSynchronize(c->stream));
+  copy_host(c->h_eq_tmp, f, nb);
+  BCK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp, nb, cudaMemcpyHostToDevice, c->stream));
   BCK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_f));
   const bool warm = opts.warm_start != 0;
   if (warm) {
-    BCK(cudaMemcpyAsync(c->d_eq_tmp, u, nb, cudaMemcpyHostToDevice, c->stream));
+    copy_host(c->h_eq_tmp + c->neq, u, nb);
+    BCK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp + c->neq, nb, cudaMemcpyHostToDevice, c->stream));
     BCK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_u));
   }
   std::vector<int32_t> it(c->nprob), dn(c->nprob);
@@ -128,8 +131,9 @@ extern "C" int fast_gpu_solve_batch(fast_gpu_ctx *c, const double *f, double *u,
   }
   c->end_span(sp);
   BCK(launch_node_to_eq(*c, c->d_u, c->d_eq_tmp));
-  BCK(cudaMemcpyAsync(u, c->d_eq_tmp, nb, cudaMemcpyDeviceToHost, c->stream));
+  BCK(cudaMemcpyAsync(c->h_eq_tmp, c->d_eq_tmp, nb, cudaMemcpyDeviceToHost, c->stream));
   BCK(cudaStreamSynchronize(c->stream));
+  copy_host(u, c->h_eq_tmp, nb);
   c->harvest();
   int bad = 0;
   for (int k = 0; k < c->nprob; k++) {

@@ -580,7 +580,13 @@ int fast_gpu_pattern_info(fast_gpu_ctx *c, int64_t *nnzb, int64_t *nnz_lower, in
 
 int fast_gpu_update_coords(fast_gpu_ctx *c, const double *coords) {
   if (check_ctx(c) || !coords || !c->d_X) return FAST_GPU_EINVAL;
-  CK(cudaMemcpyAsync(c->d_X, coords, sizeof(double) * 3 * c->nnode, cudaMemcpyHostToDevice, c->stream));
+  const double *src = coords;
+  if (c->h_eq_tmp && 3 * c->nnode <= 2 * (int64_t)c->neq) {
+    CK(cudaStreamSynchronize(c->stream));
+    copy_host(c->h_eq_tmp, coords, sizeof(double) * 3 * c->nnode);
+    src = c->h_eq_tmp;
+  }
+  CK(cudaMemcpyAsync(c->d_X, src, sizeof(double) * 3 * c->nnode, cudaMemcpyHostToDevice, c->stream));
   c->mf.geo_ok = false;
   c->K_ok = c->M_ok = false;
   invalidate(*c, FAST_ASM_STIFFNESS);
@@ -608,15 +614,14 @@ int fast_gpu_update_material(fast_gpu_ctx *c, int32_t b, const double *E, const 
     double *h = c->h_eq_tmp;
     if (E) {
       CK(cudaStreamSynchronize(c->stream));
-      for (int64_t s = 0; s < B.ne; s++) h[s] = E[B.perm[s]];
+      gather_host(h, E, B.perm.data(), B.ne);
       CK(cudaMemcpyAsync(B.d_E, h, sizeof(double) * B.ne, cudaMemcpyHostToDevice, c->stream));
     }
     if (nu) {
       CK(cudaStreamSynchronize(c->stream));
-      for (int64_t s = 0; s < B.ne; s++) h[s] = nu[B.perm[s]];
+      gather_host(h, nu, B.perm.data(), B.ne);
       CK(cudaMemcpyAsync(B.d_nu, h, sizeof(double) * B.ne, cudaMemcpyHostToDevice, c->stream));
     }
-    CK(cudaStreamSynchronize(c->stream));
   }
   c->mf.mat_ok = false;
   c->K_ok = c->M_ok = false;
@@ -635,7 +640,7 @@ int fast_gpu_set_displacement(fast_gpu_ctx *c, const double *u) {
   if (check_ctx(c) || !u || !c->d_disp) return FAST_GPU_EINVAL;
   const size_t nb = sizeof(double) * c->neq;
   CK(cudaStreamSynchronize(c->stream));
-  std::memcpy(c->h_eq_tmp, u, nb);
+  copy_host(c->h_eq_tmp, u, nb);
   CK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp, nb, cudaMemcpyHostToDevice, c->stream));
   CK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_disp));
   return FAST_GPU_OK;
@@ -661,7 +666,7 @@ int fast_gpu_internal_force(fast_gpu_ctx *c, double *g) {
   CK(cudaMemcpyAsync(c->h_eq_tmp, c->d_eq_tmp, nb, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  std::memcpy(g, c->h_eq_tmp, nb);
+  copy_host(g, c->h_eq_tmp, nb);
   if (c->h_status[0] & 1) {
     c->err = "internal_force: non-positive Jacobian determinant in at least one element";
     return FAST_GPU_EDETJ;
@@ -800,7 +805,7 @@ int fast_gpu_mult_vect(fast_gpu_ctx *c, int32_t what, const double *x, double *y
   if (!T || (what == FAST_ASM_STIFFNESS && !c->K_ok) || (what == FAST_ASM_MASS && !c->M_ok)) return FAST_GPU_ESTATE;
   const size_t nb = sizeof(double) * c->neq;
   CK(cudaStreamSynchronize(c->stream));
-  std::memcpy(c->h_eq_tmp, x, nb);
+  copy_host(c->h_eq_tmp, x, nb);
   CK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp, nb, cudaMemcpyHostToDevice, c->stream));
   CK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_z));
   // the solve layout where it is there: a product takes 112 us on it and 127 on
@@ -812,7 +817,7 @@ int fast_gpu_mult_vect(fast_gpu_ctx *c, int32_t what, const double *x, double *y
   CK(launch_node_to_eq(*c, c->d_w, c->d_eq_tmp));
   CK(cudaMemcpyAsync(c->h_eq_tmp, c->d_eq_tmp, nb, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  std::memcpy(y, c->h_eq_tmp, nb);
+  copy_host(y, c->h_eq_tmp, nb);
   return FAST_GPU_OK;
 }
 
@@ -959,14 +964,14 @@ int fast_gpu_solve(fast_gpu_ctx *c, const double *f, double *u, const fast_gpu_s
   const size_t nb = sizeof(double) * c->neq;
   double *d_feq = c->d_eq_tmp, *d_ueq = c->d_eq_tmp + c->neq;
   CK(cudaStreamSynchronize(c->stream));
-  std::memcpy(c->h_eq_tmp, f, nb);
-  if (o && o->warm_start) std::memcpy(c->h_eq_tmp + c->neq, u, nb);
+  copy_host(c->h_eq_tmp, f, nb);
+  if (o && o->warm_start) copy_host(c->h_eq_tmp + c->neq, u, nb);
   CK(cudaMemcpyAsync(d_feq, c->h_eq_tmp, (o && o->warm_start) ? 2 * nb : nb, cudaMemcpyHostToDevice, c->stream));
   const int rc = fast_gpu_solve_device(c, d_feq, d_ueq, o, rep);
   if (rc == FAST_GPU_OK || rc == FAST_GPU_ENONCONV) {
     CK(cudaMemcpyAsync(c->h_eq_tmp, d_ueq, nb, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    std::memcpy(u, c->h_eq_tmp, nb);
+    copy_host(u, c->h_eq_tmp, nb);
   }
   return rc;
 }

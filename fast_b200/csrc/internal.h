@@ -247,7 +247,7 @@ struct Ctx {
   PcgState *d_state = nullptr;
   PcgState *h_state = nullptr;    // pinned
   double *d_eq_tmp = nullptr;     // [neq] staging for host <-> device in equation space
-  double *h_eq_tmp = nullptr;     // pinned [neq]
+  double *h_eq_tmp = nullptr;     // pinned [2 neq] staging: whoever fills it synchronises the stream first
 
   // matrix-free solves (matfree.cu)
   MatFree mf;
@@ -373,6 +373,9 @@ inline int elem_per_sm(Ctx &c, int occ, int cap) {
 // pattern.cpp
 bool build_pattern(Ctx &c, const fast_gpu_mesh &m);
 
+// staging.cpp: dst = src, and dst[i] = src[at[i]], on several host threads when large
+void copy_host(void *dst, const void *src, size_t bytes);
+void gather_host(double *dst, const double *src, const int32_t *at, int64_t n);
 // shape tables (shape_tables.cpp)
 bool gauss_rule(int n, double *r, double *w);
 void gauss_point_tables(int type, const int ngp[3], std::vector<double> &N, std::vector<double> &dN,
