@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(NT, 1) bsp_elem_kernel(ElemArgs A, int split) 
   uint8_t *spair = reinterpret_cast<uint8_t *>(sWg + S::kWg);
   uint8_t *sfix = spair + 2 * NP;
   const int tid = threadIdx.x;
+  chain_release();
   for (int q = tid; q < NP; q += NT) {
     int a, b;
     pair_of(q, NN, a, b);
@@ -227,6 +228,7 @@ __global__ void __launch_bounds__(NT, 1) bsp_elem_kernel(ElemArgs A, int split) 
     const double dd = (1.0 + nu) * (1.0 - 2.0 * nu);
     const double C00 = E * (1.0 - nu) / dd, C01 = E * nu / dd, G = 0.5 * E / (1.0 + nu);
     const double rho = (MASS && A.rho) ? A.rho[e] : 0.0;
+    if (wi == blockIdx.x) chain_wait();
     for (int q = tid + part * NT; q < NP; q += NT * split) {
       const int pa = spair[2 * q], pb = spair[2 * q + 1];
       // the pair's two K blocks are loaded before its Gauss-point sum, so the
@@ -327,9 +329,8 @@ static cudaError_t run_bsp(Ctx &c, ElemArgs a, int64_t count) {
   if (a.split > 0) split = std::min(a.split, smax);
   int64_t grid = std::min<int64_t>(slots, count * split);
   a.ne = count;
-  kern<<<(unsigned)grid, NT, S::bytes, c.stream>>>(a, split);
   c.launches++;
-  return cudaGetLastError();
+  return launch_chained(a.chain, kern, dim3((unsigned)grid), dim3(NT), S::bytes, c.stream, a, split);
 }
 
 // Higher degrees (the reference's (4,2,4) and (5,2,5) NURBS cylinders): the

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(NT, (NT >= 128 ? 3 : 8)) elem_kernel(ElemArgs 
   const double *__restrict__ gw = A.w;
 
   const int tid = threadIdx.x;
+  chain_release();
   if (MASS)
     for (int i = tid; i < S::kN; i += NT) sN[i] = A.N[i];
   int pa = 0, pb = 0;
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(NT, (NT >= 128 ? 3 : 8)) elem_kernel(ElemArgs 
     }
     for (int i = tid; i < NN; i += NT) sfix[i] = A.fix[en[i]];
 
+    if (it == blockIdx.x) chain_wait();
     // early scatter loads: slots, then the current block values
     // (a block this element writes first is not read: sSlot holds ~slot for it)
     double *Kab = nullptr, *Kba = nullptr;
@@ -293,9 +295,8 @@ static cudaError_t run(Ctx &c, ElemArgs a, int64_t count) {
   int64_t grid = (int64_t)per_sm * c.sm_count;
   if (grid > count) grid = count;
   a.ne = count;
-  kern<<<(unsigned)grid, NT, S::bytes, c.stream>>>(a);
   c.launches++;
-  return cudaGetLastError();
+  return launch_chained(a.chain, kern, dim3((unsigned)grid), dim3(NT), S::bytes, c.stream, a);
 }
 
 template <bool MASS>
@@ -384,6 +385,7 @@ cudaError_t launch_tied_element_matrices(Ctx &c) {
 }
 
 cudaError_t launch_assemble(Ctx &c, int what, double *target) {
+  bool chain = false;
   for (size_t b = 0; b < c.buckets.size(); b++) {
     const Bucket &B = c.buckets[b];
     if (what == FAST_ASM_MASS && !B.has_rho) continue;
@@ -391,12 +393,14 @@ cudaError_t launch_assemble(Ctx &c, int what, double *target) {
     for (size_t k = 0; k + 1 < B.color_off.size(); k++) {
       ElemArgs a = base_args(c, B, target);
       a.offset = B.color_off[k];
+      a.chain = chain;
       if (what == FAST_ASM_STIFFNESS && c.use_first_touch()) {
         a.first = B.d_first;
         a.fw = first_words(B.nn);
       }
       const int64_t cnt = B.color_off[k + 1] - B.color_off[k];
       cudaError_t e = (what == FAST_ASM_MASS) ? dispatch<true>(c, B, a, cnt) : dispatch<false>(c, B, a, cnt);
+      chain = chain || cnt > 0;
       if (e != cudaSuccess) return e;
     }
   }

@@ -19,12 +19,13 @@
 //     up with all nine M_ij of its two pairs (a, b), (a, b+1) of each tile, so
 //     the isotropic blocks need no exchange;
 //   * the blocks go through shared memory (in D's place) and are added to the
-//     values that cp.async has fetched meanwhile, consecutive lanes taking
+//     values that cp.async fetches during the product, consecutive lanes taking
 //     consecutive entries of a block.
 // The next element's slots, flags and nodes are on their way meanwhile.  54 KB
 // and 96 threads per element: four elements per SM.
 // Measured at 32,760 hex20 elements, 27 points: 1,287 us with a thread per pair,
-// 1,157 with the entry indices worked out per entry, 1,000 like this.  Half of
+// 1,157 with the entry indices worked out per entry, 1,000 like this
+// (with the old values fetched before the Jacobians, the launches in turn).  Half of
 // it is the scatter: with the matrix instructions left out a colour takes 105 of
 // 125 us, with the scatter left out 62 (loads into registers in fifteens
 // instead of cp.async, five elements per SM: 122).
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(kT, 4) elem_mma20(ElemArgs A, const double *__
   uint8_t *sfix = reinterpret_cast<uint8_t *>(sQ + kN * kN);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   // scatter: 27 lanes of a warp take three blocks at a time, entry k of each
+  chain_release();
   const int kb = lane / 9, k9 = lane - 9 * kb, kt9 = 3 * (k9 % 3) + k9 / 3, q0 = 3 * w + kb;
   for (int q = tid; q < kN * kN; q += kT) sQ[q] = block_word(q);
   auto ahead = [&](int64_t it) {  // an element's slots, flags and nodes
@@ -135,19 +137,6 @@ __global__ void __launch_bounds__(kT, 4) elem_mma20(ElemArgs A, const double *__
       sSlot[q] = fst ? ~sRow[q] : sRow[q];
     }
     const bool any_fixed = __syncthreads_or(fixed_node);
-    if (lane < 27) {
-#pragma unroll 5
-      for (int q = q0; q < kN * kN; q += 9) {
-        const int32_t sl = sSlot[q];
-        if (sl >= 0)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                           (unsigned)__cvta_generic_to_shared(sKo + 9 * q + k9)),
-                       "l"(A.K + (int64_t)sl * 9 + k9)
-                       : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    ahead(it + gridDim.x);
     // Jacobians J[p][q] = sum_a dN_a/dxi_p X_a,q (cShapeSolid::DrvShpXYZ, shp/shpsolid.cpp:58-126)
     for (int g = lane; g < NG; g += 32) {
       double j0 = 0.0, j1 = 0.0, j2 = 0.0;
@@ -195,6 +184,20 @@ __global__ void __launch_bounds__(kT, 4) elem_mma20(ElemArgs A, const double *__
         D[48 + a] = sq * (J[6] * d0 + J[7] * d1 + J[8] * d2);
       }
     }
+    if (it == blockIdx.x) chain_wait();
+    if (lane < 27) {
+#pragma unroll 5
+      for (int q = q0; q < kN * kN; q += 9) {
+        const int32_t sl = sSlot[q];
+        if (sl >= 0)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(sKo + 9 * q + k9)),
+                       "l"(A.K + (int64_t)sl * 9 + k9)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ahead(it + gridDim.x);
     const double E = A.E[e], nu = A.nu[e];
     __syncthreads();
     double M[2][9][2];
@@ -265,9 +268,9 @@ cudaError_t run(Ctx &c, const Bucket &B, ElemArgs a, int64_t count) {
   if (e != cudaSuccess) return e;
   per_sm = elem_per_sm(c, per_sm, a.ctas_per_sm);
   a.ne = count;
-  kern<<<(unsigned)std::min<int64_t>((int64_t)per_sm * c.sm_count, count), kT, bytes, c.stream>>>(a, B.d_dNt);
   c.launches++;
-  return cudaGetLastError();
+  return launch_chained(a.chain, kern, dim3((unsigned)std::min<int64_t>((int64_t)per_sm * c.sm_count, count)), dim3(kT),
+                        bytes, c.stream, a, B.d_dNt);
 }
 
 }  // namespace

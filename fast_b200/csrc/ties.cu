@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kTiedThreads) tied_scatter(int64_t first, int6
                              const int64_t *__restrict__ keoff, const int32_t *__restrict__ nn_of,
                              const double *__restrict__ ke, const uint8_t *__restrict__ fix, KT *__restrict__ K) {
   extern __shared__ double sKe[];
+  chain_release();
   for (int64_t it = blockIdx.x; it < count; it += gridDim.x) {
     const int64_t x = first + it;
     const int64_t n0 = nptr[x];
@@ -53,7 +54,8 @@ __global__ void __launch_bounds__(kTiedThreads) tied_scatter(int64_t first, int6
       Ke = sKe;
     }
     const int32_t *sl = slot + sptr[x];
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
+    if (it == blockIdx.x) chain_wait();
+    for (int q = threadIdx.x + blockIdx.y * blockDim.x; q < m * m; q += blockDim.x * gridDim.y) {
       const int A = q / m, B = q - A * m;
       double v[9];
 #pragma unroll
@@ -225,28 +227,29 @@ template <typename KT>
 static cudaError_t tied_scatter_all(Ctx &c, KT *K) {
   TiedSet &T = c.tied;
   cudaError_t e = cudaSuccess;
+  bool chain = false;
   for (size_t k = 0; k + 1 < T.color_off.size(); k++) {
     const int64_t first = T.color_off[k], cnt = T.color_off[k + 1] - first;
     if (cnt <= 0) continue;
-    // one element per CTA; 1024 threads share its expanded pairs, whose K
-    // read-modify-writes are latency-bound
-    const unsigned grid = (unsigned)std::min<int64_t>(cnt, 2LL * c.sm_count);
+    // an element's expanded pairs, whose K read-modify-writes are latency-bound,
+    // go to as many CTAs of 1024 threads as fill the chip, eight at most
+    const unsigned gx = (unsigned)std::min<int64_t>(cnt, 2LL * c.sm_count);
+    const dim3 grid(gx, (unsigned)std::max<int64_t>(1, std::min<int64_t>(8, 2LL * c.sm_count / gx)));
     int maxnn = 0;
     for (int32_t v : T.h_nn) maxnn = std::max(maxnn, v);
-    const size_t smem = sizeof(double) * 9 * maxnn * maxnn;
+    size_t smem = sizeof(double) * 9 * maxnn * maxnn;
+    auto kern = tied_scatter<true, KT>;
     if (smem <= 96 * 1024) {
-      e = cudaFuncSetAttribute(tied_scatter<true, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      tied_scatter<true, KT><<<grid, kTiedThreads, smem, c.stream>>>(first, cnt, T.d_nptr, T.d_nodes, T.d_sptr,
-                                                                      T.d_slot, T.d_pptr, T.d_pa, T.d_pt, T.d_keoff,
-                                                                      T.d_nn, T.d_ke, c.d_fix, K);
     } else {
-      tied_scatter<false, KT><<<grid, kTiedThreads, 0, c.stream>>>(first, cnt, T.d_nptr, T.d_nodes, T.d_sptr, T.d_slot,
-                                                                    T.d_pptr, T.d_pa, T.d_pt, T.d_keoff, T.d_nn,
-                                                                    T.d_ke, c.d_fix, K);
+      kern = tied_scatter<false, KT>;
+      smem = 0;
     }
+    e = launch_chained(chain, kern, grid, dim3(kTiedThreads), smem, c.stream, first, cnt, T.d_nptr, T.d_nodes, T.d_sptr,
+                       T.d_slot, T.d_pptr, T.d_pa, T.d_pt, T.d_keoff, T.d_nn, T.d_ke, c.d_fix, K);
+    chain = true;
     c.launches++;
-    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

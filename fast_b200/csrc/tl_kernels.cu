@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(NT, (NT >= 128 ? 3 : 8)) tl_kernel(ElemArgs A)
   const double *__restrict__ gdN = A.dN;
   const double *__restrict__ gw = A.w;
   const int tid = threadIdx.x;
+  chain_release();
   int pa = 0, pb = 0;
   if (tid < NP) pair_of(tid, NN, pa, pb);
 
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(NT, (NT >= 128 ? 3 : 8)) tl_kernel(ElemArgs A)
     }
     for (int i = tid; i < NN; i += NT) sfix[i] = A.fix[en[i]];
 
+    if (it == blockIdx.x) chain_wait();
     double *Kab = nullptr, *Kba = nullptr;
     double oab[9], oba[9];
     if (WANT_K && A.K && tid < NP) {
@@ -305,9 +307,8 @@ static cudaError_t run_tl(Ctx &c, ElemArgs a, int64_t count) {
   int64_t grid = (int64_t)per_sm * c.sm_count;
   if (grid > count) grid = count;
   a.ne = count;
-  kern<<<(unsigned)grid, NT, S_::bytes, c.stream>>>(a);
   c.launches++;
-  return cudaGetLastError();
+  return launch_chained(a.chain, kern, dim3((unsigned)grid), dim3(NT), S_::bytes, c.stream, a);
 }
 
 // mode: 0 tangent + internal force, 1 tangent only, 2 internal force only
@@ -401,6 +402,7 @@ cudaError_t launch_tl_at(Ctx &c, double *K, double *G, bool want_k, bool want_g,
     c.launches++;
     return cudaGetLastError();
   }
+  bool chain = false;
   for (size_t b = 0; b < c.buckets.size(); b++) {
     const Bucket &B = c.buckets[b];
     int mode;
@@ -416,7 +418,9 @@ cudaError_t launch_tl_at(Ctx &c, double *K, double *G, bool want_k, bool want_g,
       a.U = U;
       a.skip = skip;
       a.offset = B.color_off[k];
+      a.chain = chain;
       const int64_t cnt = B.color_off[k + 1] - B.color_off[k];
+      chain = chain || cnt > 0;
       cudaError_t e = B.type == FAST_ELEM_BSP_SOLID ? launch_bsp_tl(c, B, a, cnt, mode)
                       : B.tl                         ? dispatch_tl<true>(c, B, a, cnt, mode)
                                                      : dispatch_tl<false>(c, B, a, cnt, mode);
