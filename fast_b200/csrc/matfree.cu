@@ -32,6 +32,7 @@
 #include <cmath>
 #include <vector>
 
+#include "elem_common.cuh"
 #include "matfree_math.cuh"
 #include "solve_common.cuh"
 
@@ -658,7 +659,7 @@ mf_residual(int64_t nnode, const int32_t *__restrict__ ptr, const int32_t *__res
 // The chip is filled whatever the mix of sizes, and nothing streams a matrix
 // (3.4 GB an iteration for 256 cantilevers with 1.8 million nodes).  There:
 // elements 183 us on average over the solve, nodes 143 (at 5.4 TB/s), alpha and
-// beta 4.8 and 3.9; all problems 780 -> 236 ms.  (The last tile of a problem
+// beta 4.8 and 3.9; all problems 780 -> 225 ms.  (The last tile of a problem
 // forming alpha or beta behind a fence and a counter: 317 instead of 268 ms for
 // assembly and solve.)
 struct MfBatch {
@@ -687,6 +688,9 @@ __global__ void __launch_bounds__(kT8, 2) mf_batch_elements(MfArgs<double> A, Mf
   } h;
   const int step = gridDim.x * (kT8 / 32);
   int b = blockIdx.x * (kT8 / 32) + (tid >> 5), k2 = 0;
+  if (b < A.nb) h.e.load(A, b, lane);
+  chain_wait();
+  chain_release();
   if (b < A.nb) h.load(A, B, b, B.bprob[b], lane);
   if (b + step < A.nb) k2 = B.bprob[b + step];
   while (b < A.nb) {
@@ -706,6 +710,8 @@ __global__ void __launch_bounds__(kT8, 2) mf_batch_elements(MfArgs<double> A, Mf
 __global__ void __launch_bounds__(128) mf_batch_alpha(MfBatch B) {
   __shared__ double sbuf[32];
   MfProblem *S = B.S + blockIdx.x;
+  chain_wait();
+  chain_release();
   if (S->done) return;
   double v = 0.0;
   for (int i = B.eptr[blockIdx.x] + threadIdx.x; i < B.eptr[blockIdx.x + 1]; i += 128) v += B.part_pw[i];
@@ -726,6 +732,8 @@ mf_batch_update(const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc
   __shared__ double sbuf[32];
   const int4 t = B.ntile[blockIdx.x];
   const MfProblem *S = B.S + t.z;
+  chain_wait();
+  chain_release();
   if (S->done) return;
   const double alpha = S->alpha, beta = S->beta;
   const int64_t n = t.x + (int)threadIdx.x;
@@ -743,6 +751,8 @@ mf_batch_update(const int32_t *__restrict__ ptr, const int32_t *__restrict__ inc
 __global__ void __launch_bounds__(128) mf_batch_beta(MfBatch B, double tol, int maxit) {
   __shared__ double sbuf[32];
   MfProblem *S = B.S + blockIdx.x;
+  chain_wait();
+  chain_release();
   if (S->done) return;
   double a = 0.0, b = 0.0;
   for (int i = B.nptr[blockIdx.x] + threadIdx.x; i < B.nptr[blockIdx.x + 1]; i += 128) {
@@ -1003,11 +1013,10 @@ bool mf_active(const Ctx &c) {
 // 1 to 1,000 cantilevers of 45 to 18,081 nodes each: an iteration of pcg_batch
 // takes 6.5 us and 0.036 us per node of its problem, 148 clusters run at once
 // and the largest problem may be what is waited for; a lockstep iteration takes
-// 24 us (four kernels) and 0.15 ns per node of all problems.  Measured, ms
-// (pcg_batch / lockstep): 8 problems of 112..637 nodes 5.6 / 5.1, 16 of 112..396
-// 3.1 / 4.3, 64 of 45..112 1.1 / 2.9, 128 of 112..637 6.5 / 6.3, 256 of 225..1,377
-// 26 / 16, 1,000 of 45 3.8 / 3.3, 8 of 1,900..18,081 501 / 23, 256 of
-// 637..18,081 780 / 236.
+// 17 us (four kernels) and 0.15 ns per node of all problems.  Measured, ms
+// (pcg_batch / lockstep): 8 problems of 112..637 nodes 5.7 / 3.5, 16 of 112..396
+// 3.1 / 3.0, 64 of 112..225 1.9 / 2.5, 128 of 112..637 6.3 / 4.7, 256 of
+// 225..1,377 26 / 14, 8 of 1,900..18,081 501 / 23, 256 of 637..18,081 780 / 225.
 bool mf_batch_active(const Ctx &c) {
   if (c.nprob <= 0 || !mf_possible(c) || c.buckets[0].nn != 8) return false;
   if (c.mf_min_nodes >= 0) return c.nnode >= c.mf_min_nodes;
@@ -1017,7 +1026,7 @@ bool mf_batch_active(const Ctx &c) {
     sum += t;
     most = std::max(most, t);
   }
-  return 24.0 + 0.15e-3 * (double)c.nnode < std::max(most, sum / c.sm_count);
+  return 17.0 + 0.15e-3 * (double)c.nnode < std::max(most, sum / c.sm_count);
 }
 
 // The batches: elements in the mesh's own order, 32 at a time; of a context with
@@ -1249,11 +1258,14 @@ cudaError_t mf_solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it
     a.nb = M.h_eptr[live];
     const int G = std::max(1, std::min(M.per_sm64 * c.sm_count, (a.nb + kT8 / 32 - 1) / (kT8 / 32)));
     for (int i = 0; i < chunk; i++) {
-      mf_batch_elements<<<G, kT8, 0, c.stream>>>(a, b);
-      mf_batch_alpha<<<live, 128, 0, c.stream>>>(b);
-      mf_batch_update<<<M.h_ntile[live], kVecThreads, 0, c.stream>>>(
-          M.ptr, M.inc, M.F64, c.d_fix, c.d_u, c.d_r, c.d_z, c.d_p, M.jacobi ? M.dj64 : nullptr, c.d_dinv, b);
-      mf_batch_beta<<<live, 128, 0, c.stream>>>(b, tol, maxit);
+      // (each is scheduled while the one before it drains: 257 -> 251 ms for the
+      // 256 cantilevers; the same in the captured chunks of a single solve was
+      // slower, 18.4 -> 20.0 ms for hex8 61x47x33)
+      launch_chained(i > 0, mf_batch_elements, G, kT8, 0, c.stream, a, b);
+      launch_chained(true, mf_batch_alpha, live, 128, 0, c.stream, b);
+      launch_chained(true, mf_batch_update, M.h_ntile[live], kVecThreads, 0, c.stream, M.ptr, M.inc, M.F64, c.d_fix, c.d_u,
+                     c.d_r, c.d_z, c.d_p, M.jacobi ? M.dj64 : nullptr, c.d_dinv, b);
+      launch_chained(true, mf_batch_beta, live, 128, 0, c.stream, b, tol, maxit);
       c.launches += 4;
     }
     if ((e = cudaGetLastError()) != cudaSuccess ||
