@@ -406,21 +406,6 @@ __global__ void __launch_bounds__(kT8) mf_hex8_32(MfArgs<float> A) {
   if (DIR) commit_direction(A.st, done, rr, zr, err, bt);
 }
 
-// A = det J J^-1 from J (J[3 c + d] = dx_c/dxi_d); returns det J
-template <typename T>
-__device__ __forceinline__ T cofactors(const T *J, T *A) {
-  A[0] = J[4] * J[8] - J[5] * J[7];
-  A[1] = J[2] * J[7] - J[1] * J[8];
-  A[2] = J[1] * J[5] - J[2] * J[4];
-  A[3] = J[5] * J[6] - J[3] * J[8];
-  A[4] = J[0] * J[8] - J[2] * J[6];
-  A[5] = J[2] * J[3] - J[0] * J[5];
-  A[6] = J[3] * J[7] - J[4] * J[6];
-  A[7] = J[1] * J[6] - J[0] * J[7];
-  A[8] = J[0] * J[4] - J[1] * J[3];
-  return J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
-}
-
 // FP64 forces of a lane's hex8 element at x = z + beta p (DIR) or p, into
 // F[node][32][4]; returns x . K_e x.  The geometry is rebuilt from the nodes'
 // coordinates (in L1 and L2: neighbours share them): 72 stored numbers a
@@ -476,7 +461,7 @@ __device__ __forceinline__ double hex8_forces(const int32_t (&n)[8], const doubl
     for (int c = 0; c < 3; c++)
 #pragma unroll
       for (int d = 0; d < 3; d++) P[3 * c + d] = sJ[(12 * c + 4 * d + id[d]) * kT8];
-    const double q = 1.0 / cofactors(P, A);
+    const double q = 1.0 / mf::cofactors(P, A);
 #pragma unroll
     for (int c = 0; c < 3; c++)
 #pragma unroll
@@ -869,7 +854,7 @@ __global__ void mf_material(int64_t n32, double scale, const int32_t *__restrict
 
 // A = sqrt(w / det J) det J J^-1 from J (det > 0: the assembly has checked it)
 __device__ __forceinline__ void point_geometry(const double *J, double w, double *A) {
-  const double s = sqrt(w / cofactors(J, A));
+  const double s = sqrt(w / mf::cofactors(J, A));
 #pragma unroll
   for (int q = 0; q < 9; q++) A[q] *= s;
 }

@@ -266,6 +266,21 @@ FG_HD void line_gradients_t(const T (*P)[9], T (*R)[8]) {
   }
 }
 
+// A = det J J^-1 from J (J[3 c + d] = dx_c/dxi_d); returns det J
+template <typename T>
+FG_HD T cofactors(const T *J, T *A) {
+  A[0] = J[4] * J[8] - J[5] * J[7];
+  A[1] = J[2] * J[7] - J[1] * J[8];
+  A[2] = J[1] * J[5] - J[2] * J[4];
+  A[3] = J[5] * J[6] - J[3] * J[8];
+  A[4] = J[0] * J[8] - J[2] * J[6];
+  A[5] = J[2] * J[3] - J[0] * J[5];
+  A[6] = J[3] * J[7] - J[4] * J[6];
+  A[7] = J[1] * J[6] - J[0] * J[7];
+  A[8] = J[0] * J[4] - J[1] * J[3];
+  return J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
+}
+
 // hex8, one component: nodal values -> the derivatives, each of which is
 // constant along its own direction: D[0] = d/dx at (y, z) signs 2 bits
 // (y + 2 z), D[1] = d/dy at x + 2 z, D[2] = d/dz at x + 2 y

@@ -23,6 +23,7 @@
 #include <cstdint>
 
 #include "elem_common.cuh"
+#include "matfree_math.cuh"
 #include "internal.h"
 
 namespace fastgpu {
@@ -293,6 +294,125 @@ __global__ void __launch_bounds__(NT, (NT >= 128 ? 3 : 8)) tl_kernel(ElemArgs A)
   }
 }
 
+// Internal force alone of hex8 elements with 2x2x2 points (all weights 1): a
+// thread per element.  64 threads and eight barrier-separated phases an
+// element, most of them idle in each, took 110 us for 38,394 elements; here
+// the gradients at the points come from sums and differences of the nodal
+// values (matfree_math.cuh), those of the coordinates waiting in the thread's
+// column of shared memory: 15 us, two blocks of 242 registers per SM.
+constexpr int kForceThreads = 128;
+
+template <bool TL>
+__global__ void __launch_bounds__(kForceThreads, 2) tl_force8(ElemArgs A) {
+  __shared__ double sJ[36 * kForceThreads];
+  chain_release();
+  const int64_t it = blockIdx.x * (int64_t)kForceThreads + threadIdx.x;
+  if (it < A.ne && !(A.skip && *A.skip)) {
+    const int64_t e = A.index ? (int64_t)A.index[it] : A.offset + it;
+    double *J = sJ + threadIdx.x;
+    const int4 c0 = reinterpret_cast<const int4 *>(A.conn + 8 * e)[0], c1 = reinterpret_cast<const int4 *>(A.conn + 8 * e)[1];
+    const int32_t n[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    const double Ey = A.E[e], nu = A.nu[e];
+    const double lam = Ey * nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu2 = Ey / (1.0 + nu);
+    double D[3][3][4], R[3][3][4];
+    {
+      double x[3][8], u[3][8];
+#pragma unroll
+      for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          x[c][a] = A.X[3 * (int64_t)n[a] + c];
+          u[c][a] = A.U[4 * (int64_t)n[a] + c];
+        }
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        mf::hex8_grads(x[c], D[c]);
+#pragma unroll
+        for (int i = 0; i < 12; i++) J[(12 * c + i) * kForceThreads] = D[c][i / 4][i % 4];
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) mf::hex8_grads(u[c], D[c]);
+    }
+#pragma unroll
+    for (int i = 0; i < 36; i++) R[i / 12][(i / 4) % 3][i % 4] = 0.0;
+    bool bad = false;
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+      const int gx = g & 1, gy = (g >> 1) & 1, gz = g >> 2;
+      const int id[3] = {gy + 2 * gz, gx + 2 * gz, gx + 2 * gy};
+      double P[9], C[9], h[9], S[6];
+#pragma unroll
+      for (int k = 0; k < 9; k++) P[k] = J[(4 * k + id[k % 3]) * kForceThreads];
+      const double det = mf::cofactors(P, C);  // C = det J J^-1
+      bad = bad || !(det > 0.0);
+      const double q = 1.0 / (det != 0.0 ? det : 1.0);
+      // displacement gradient h_ij = du_i/dX_j
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+          h[3 * i + j] = q * (D[i][0][id[0]] * C[j] + D[i][1][id[1]] * C[3 + j] + D[i][2][id[2]] * C[6 + j]);
+      // strain (TL: F^T F = I + h + h^T + h^T h), stress S = lambda tr(E) I + 2 mu E: xx yy zz xy xz yz
+      double E[6] = {h[0], h[4], h[8], 0.5 * (h[1] + h[3]), 0.5 * (h[2] + h[6]), 0.5 * (h[5] + h[7])};
+      if (TL) {
+        E[0] += 0.5 * (h[0] * h[0] + h[3] * h[3] + h[6] * h[6]);
+        E[1] += 0.5 * (h[1] * h[1] + h[4] * h[4] + h[7] * h[7]);
+        E[2] += 0.5 * (h[2] * h[2] + h[5] * h[5] + h[8] * h[8]);
+        E[3] += 0.5 * (h[0] * h[1] + h[3] * h[4] + h[6] * h[7]);
+        E[4] += 0.5 * (h[0] * h[2] + h[3] * h[5] + h[6] * h[8]);
+        E[5] += 0.5 * (h[1] * h[2] + h[4] * h[5] + h[7] * h[8]);
+      }
+      const double tr = lam * (E[0] + E[1] + E[2]);
+#pragma unroll
+      for (int k = 0; k < 6; k++) S[k] = mu2 * E[k] + (k < 3 ? tr : 0.0);
+      // P = F S (TL) or S; its part of R is P_ij C_dj
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        double p0 = S[i == 0 ? 0 : (i == 1 ? 3 : 4)], p1 = S[i == 0 ? 3 : (i == 1 ? 1 : 5)],
+               p2 = S[i == 0 ? 4 : (i == 1 ? 5 : 2)];
+        if (TL) {
+          const double h0 = h[3 * i], h1 = h[3 * i + 1], h2 = h[3 * i + 2];
+          p0 += h0 * S[0] + h1 * S[3] + h2 * S[4];
+          p1 += h0 * S[3] + h1 * S[1] + h2 * S[5];
+          p2 += h0 * S[4] + h1 * S[5] + h2 * S[2];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) R[i][d][id[d]] += p0 * C[3 * d] + p1 * C[3 * d + 1] + p2 * C[3 * d + 2];
+      }
+    }
+    if (bad) atomicOr(A.status, 1);
+    double f[3][8];
+#pragma unroll
+    for (int c = 0; c < 3; c++) mf::hex8_grads_t(R[c], f[c]);
+    chain_wait();
+    if (A.G) {
+#pragma unroll
+      for (int a = 0; a < 8; a++) {
+        const uint8_t m = A.fix[n[a]];
+        double *Gn = A.G + 4 * (int64_t)n[a];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          if (!((m >> c) & 1)) Gn[c] += f[c][a];
+      }
+    }
+    if (A.Ke_out) {
+      double2 *Go = reinterpret_cast<double2 *>(A.Ke_out + it * 24);
+#pragma unroll
+      for (int k = 0; k < 12; k++)
+        Go[k] = make_double2(f[(2 * k) % 3][(2 * k) / 3], f[(2 * k + 1) % 3][(2 * k + 1) / 3]);
+    }
+  }
+}
+
+template <bool TL>
+static cudaError_t run_force8(Ctx &c, ElemArgs a, int64_t count) {
+  if (count <= 0) return cudaSuccess;
+  a.ne = count;
+  c.launches++;
+  return launch_chained(a.chain, tl_force8<TL>, dim3((unsigned)((count + kForceThreads - 1) / kForceThreads)),
+                        dim3(kForceThreads), 0, c.stream, a);
+}
+
 template <int NN, int NG, int NT, bool TL, bool WK, bool WG>
 static cudaError_t run_tl(Ctx &c, ElemArgs a, int64_t count) {
   if (count <= 0) return cudaSuccess;
@@ -320,7 +440,10 @@ static cudaError_t dispatch_tl(Ctx &c, const Bucket &B, ElemArgs a, int64_t coun
   if (mode == 1) return run_tl<NN, NG, NT, TL, true, false>(c, a, count);                   \
   return run_tl<NN, NG, NT, TL, false, true>(c, a, count);
   if (B.type == FAST_ELEM_HEX8) {
-    if (ng == 8) { FASTGPU_TL_CASES(8, 8, 64) }
+    if (ng == 8) {
+      if (mode == 2) return run_force8<TL>(c, a, count);
+      return mode == 0 ? run_tl<8, 8, 64, TL, true, true>(c, a, count) : run_tl<8, 8, 64, TL, true, false>(c, a, count);
+    }
     if (ng == 27) { FASTGPU_TL_CASES(8, 27, 64) }
     if (ng == 1) { FASTGPU_TL_CASES(8, 1, 64) }
   } else if (B.type == FAST_ELEM_HEX20) {

@@ -95,3 +95,28 @@ def test_mass_reports_an_inverted_element():
         s.assemble_mass()
     s.update_coords(d.coords)
     s.assemble_mass()
+
+
+@pytest.mark.parametrize("gather", [0, 1])
+@pytest.mark.parametrize("tl", [False, True])
+@pytest.mark.parametrize("mesh", [(1, 1, 1), (5, 4, 3), (16, 8, 1), (43, 3, 1), "wheel"])
+def test_hex8_internal_force_matches_oracle(mesh, tl, gather):
+    """Around a block of 128 elements, per node and colour by colour."""
+    d = _deck("hex8", 2, mesh)
+    d.total_lagrangian = tl
+    rng = np.random.default_rng(7)
+    u = 0.05 * rng.standard_normal(d.num_eq())
+    eq = d.node_eq()
+    full = np.where(eq > 0, u[np.maximum(eq, 1) - 1], 0.0)
+    want, size = np.zeros(d.num_eq() + 1), np.zeros(d.num_eq() + 1)
+    for e, en in enumerate(d.conn):
+        f = (fo.elem_tl if tl else fo.elem_intforce)(8, d.ngp, d.coords[en], d.E[e], d.nu[e], full[en].ravel())
+        g = np.asarray([v for v in f if np.ndim(v) == 1 and np.size(v) == 24][0])
+        np.add.at(want, eq[en].ravel(), g)
+        np.add.at(size, eq[en].ravel(), np.abs(g))
+    s = gpu.GpuSystem(0)
+    s.upload(d)
+    s.set_option(gpu.OPT_FORCE_GATHER, gather)
+    s.set_displacement(u)
+    got = s.internal_force()
+    assert np.abs(got - want[1:]).max() <= TOL * size[1:].max()
