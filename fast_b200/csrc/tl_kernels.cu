@@ -324,6 +324,14 @@ __global__ void __launch_bounds__(kForceThreads, 2) tl_force8(ElemArgs A) {
           x[c][a] = A.X[3 * (int64_t)n[a] + c];
           u[c][a] = A.U[4 * (int64_t)n[a] + c];
         }
+      // relative to the first node: the element's size, not its place, bounds the rounding
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int a = 7; a >= 0; a--) {
+          x[c][a] -= x[c][0];
+          u[c][a] -= u[c][0];
+        }
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         mf::hex8_grads(x[c], D[c]);
