@@ -697,8 +697,12 @@ def run_reference(args):
     return 0
 
 
-def spmv_kernel_name(tune, which):
-    """The SpMV form the autotuner left in place for the timed solve."""
+def spmv_kernel_name(tune, which, matrix_free=False):
+    """The form of K.p in the timed solve: element by element, or the SpMV that
+    the autotuner left in place."""
+    if matrix_free:
+        return "mf_hex20<%s> (K.p element by element; the bytes are the operator's, mf_update has its own)" % (
+            "float" if which == gpu_const("KERNEL_SPMV_FP32") else "double")
     if which != gpu_const("KERNEL_SPMV_FP32"):
         return "spmv_f64<0, %d> (FP64 PCG K.p)" % tune["lanes_fp64"]
     if tune.get("col16_fp32"):
@@ -798,6 +802,8 @@ def run_ours(args):
     its = sum(r["iterations"] for r in reps_t)
     outs = sum(r["outer"] for r in reps_t)
     k_span, k_tot, k_bytes = S.kernel_stats(spmv_which)
+    # the assembled matrix is at least 36 bytes a block
+    matrix_free = k_bytes < 20.0 * S.pattern_info()["nnz_blocks"]
     k_n = its
     k_ms = k_tot / k_n
     r_span, r_tot, r_bytes = S.kernel_stats(gpu.KERNEL_SPMV_FP64)
@@ -895,7 +901,7 @@ def run_ours(args):
     a_gbs = a_bytes / (a_ms / 1e3) / 1e9 if a_ms > 0 else 0.0
     traffic = None
     tp = os.path.join(ROOT, "profiles", spmv_profile_file(tune, spmv_which))
-    if os.path.exists(tp):
+    if os.path.exists(tp) and not matrix_free:
         for ln in open(tp):
             if ln.startswith("dram_bytes_per_launch:"):
                 traffic = float(ln.split(":")[1])
@@ -970,7 +976,7 @@ def run_ours(args):
             "config": workload_config(args, neq),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm, "traffic": traffic,
-                         "kernel": spmv_kernel_name(tune, spmv_which),
+                         "kernel": spmv_kernel_name(tune, spmv_which, matrix_free),
                          "bytes_per_launch": k_bytes, "ms_per_launch": k_ms, "launches_timed": k_n,
                          "spans_timed": k_span,
                          "peak_kind": hbm_kind},
@@ -980,7 +986,7 @@ def run_ours(args):
             "clocks": clk,
             "spmv_fp64_in_timed_region": ({"launches": r_n, "ms_per_launch": r_ms, "spans": r_span,
                                            "GB_per_s": r_bytes / (r_ms / 1e3) / 1e9 if r_ms else None}
-                                          if spmv_which != gpu.KERNEL_SPMV_FP64 else None),
+                                          if spmv_which != gpu.KERNEL_SPMV_FP64 and r_span else None),
             "u_rel_err_vs_oracle": oracle["value_path"]["u_rel_err_vs_oracle"] if oracle else None,
             "solve": {"iterations": last["iterations"], "outer": last["outer"], "escalated": last["escalated"],
                       "rel_residual": last["rel_residual"], "true_rel_residual": last["true_rel_residual"],

@@ -1127,11 +1127,14 @@ int fast_gpu_kernel_stats(fast_gpu_ctx *c, int32_t which, int64_t *launches, dou
     if (which == FAST_KERNEL_SPMV_FP32)
       algo = c->spmv32_c16 ? (double)c->nnzb * (9 * 4 + 2) + 4.0 * (c->nnode + 1) + 4.0 * c->nnode + 2.0 * 4 * n4
                            : (double)c->nnzb * (9 * 4 + 4) + 4.0 * (c->nnode + 1) + 2.0 * 4 * n4;
-    // matrix-free solves: incidence, geometry, lambda and mu, the direction (with z) and the element forces once each
+    // matrix-free solves: incidence, geometry (FP64 hex8: the coordinates), lambda and mu, the direction (with z) and the
+    // element forces once each
     if (c->mf_used && (which == FAST_KERNEL_SPMV_FP64 || which == FAST_KERNEL_SPMV_FP32)) {
       const Bucket &B = c->buckets[0];
       const double t = which == FAST_KERNEL_SPMV_FP64 ? 8.0 : 4.0;
-      algo = (double)B.ne * (4.0 * B.nn + t * (9.0 * B.ng + 2.0 + 3.0 * B.nn)) + 2.0 * t * n4;
+      const bool stored = B.nn == 20 || t == 4.0;
+      algo = (double)B.ne * (4.0 * B.nn + t * ((stored ? 9.0 * B.ng : 0.0) + 2.0 + 3.0 * B.nn)) + 2.0 * t * n4 +
+             (stored ? 0.0 : 24.0 * c->nnode);
     }
     if (which == FAST_KERNEL_ASSEMBLE || which == FAST_KERNEL_ASSEMBLE_TF32) {
       // scatter model per element: incidence + coordinates + fixity + E, nu + slot map + 3x3 block

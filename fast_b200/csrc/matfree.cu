@@ -30,6 +30,7 @@
 // is one full line per warp.
 #include <algorithm>
 #include <cmath>
+#include <new>
 #include <vector>
 
 #include "elem_common.cuh"
@@ -1053,7 +1054,7 @@ static void mf_slots(Ctx &c, std::vector<int32_t> &at, std::vector<int32_t> &slo
 }
 
 // the batched copies of mesh, geometry and material, whichever are stale
-cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
+static cudaError_t prepare(Ctx &c, bool fp32, int precond) {
   MatFree &M = c.mf;
   const Bucket &B = c.buckets[0];
   const int64_t ne = B.ne, nn = B.nn;
@@ -1164,6 +1165,14 @@ cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
   return cudaGetLastError();
 }
 
+cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
+  try {
+    return prepare(c, fp32, precond);
+  } catch (const std::bad_alloc &) {
+    return cudaErrorMemoryAllocation;
+  }
+}
+
 template <typename T>
 void mf_iterations(Ctx &c, int k, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr) {
   const MatFree &M = c.mf;
@@ -1202,7 +1211,7 @@ cudaError_t mf_residual_of(Ctx &c, const double *f, const double *u, double *r, 
 // Per-problem PCG of every problem, as launch_pcg_batch.  The problems lie
 // largest first, so the launches shrink from the end as the small ones, which
 // need fewer iterations, are done.
-cudaError_t mf_solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it, double *err, int32_t *done) {
+static cudaError_t solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it, double *err, int32_t *done) {
   MatFree &M = c.mf;
   cudaError_t e;
   const int np = c.nprob;
@@ -1266,6 +1275,14 @@ cudaError_t mf_solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it
     done[c.h_order[k]] = S[k].done;
   }
   return cudaSuccess;
+}
+
+cudaError_t mf_solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t *it, double *err, int32_t *done) {
+  try {
+    return solve_batch(c, tol, maxit, warm, it, err, done);
+  } catch (const std::bad_alloc &) {
+    return cudaErrorMemoryAllocation;
+  }
 }
 
 }  // namespace fastgpu

@@ -120,3 +120,29 @@ def test_hex8_internal_force_matches_oracle(mesh, tl, gather):
     s.set_displacement(u)
     got = s.internal_force()
     assert np.abs(got - want[1:]).max() <= TOL * size[1:].max()
+
+
+def test_large_host_arrays_arrive_whole():
+    """Copies of more than 3 MB are shared among threads: a system updated to
+    other moduli and coordinates equals one uploaded with them, bit for bit."""
+    import dataclasses
+    rng = np.random.default_rng(3)
+    X, conn, _ = decks.box_mesh("hex8", (75, 74, 73), (75.0, 74.0, 73.0))
+    fixed = np.zeros(X.shape, bool)
+    fixed[X[:, 0] < 1e-9] = True
+    ne = len(conn)
+    d = decks.Deck("hex8", X, conn, np.full(ne, 1000.0), np.full(ne, 0.3), (2, 2, 2), fixed, matrix_type="sparse")
+    assert 8 * ne > 3 << 20
+    E, X2 = rng.uniform(500.0, 2000.0, ne), X + rng.uniform(-0.05, 0.05, X.shape)
+    x = rng.standard_normal(d.num_eq())
+    y = []
+    for upd in (True, False):
+        s = gpu.GpuSystem(0)
+        s.upload(d if upd else dataclasses.replace(d, E=E, coords=X2))
+        if upd:
+            s.update_material(E)
+            s.update_coords(X2)
+        s.assemble()
+        y.append(s.mult_vect(x))
+        s.close()
+    assert y[0].tobytes() == y[1].tobytes() and np.abs(y[0]).min() >= 0.0 and np.isfinite(y[0]).all()
