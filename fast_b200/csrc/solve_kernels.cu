@@ -38,6 +38,7 @@
 
 #include <cooperative_groups.h>
 
+#include "grid_scale.h"
 #include "internal.h"
 #include "solve_common.cuh"
 
@@ -1170,14 +1171,6 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ double pow2(int e) {  // 2^e, |e| <= 1022
-  return __longlong_as_double((long long)(e + 1023) << 52);
-}
-__device__ __forceinline__ double scale2(double x, int e) {  // x 2^e for |e| <= 2044 in two steps
-  const int h = e / 2;
-  return x * pow2(h) * pow2(e - h);
-}
-
 // Sum over the grid of NV values per thread, the same bits in every block.
 // With ORDERED it is a barrier too: what any thread wrote before it is visible
 // to every thread after it; without, only the sums are exchanged.
@@ -1189,7 +1182,8 @@ __device__ __forceinline__ double scale2(double x, int e) {  // x 2^e for |e| <=
 // independent of the order of arrival (and exact).  E follows the last value
 // of the same sum (ref) with 40 bits of headroom, which leaves 90 bits below
 // it; a value that does not fit adds a mark instead, and a sum that leaves
-// less than 64 bits is formed again: all blocks see the same words and repeat
+// less than 64 bits is formed again, a bounded number of times (grid_scale.h:
+// limbs, marks and the choice of E): all blocks see the same words and repeat
 // with the same E.  The words are never reset: a block remembers what it saw.
 // The two sets alternate, so a block cannot add to a word that another block
 // still waits for.  Measured on 148 blocks (cycles): release counter and
@@ -1238,13 +1232,11 @@ __device__ bool grid_sum(GridSlots *S, SumShared &sh, int CS, int rank, SumState
   }
   if (wid == 0) {
     double t[NV], res[NV];
-    int E[NV];
+    SumScale E[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) {
       t[k] = warp_sum(lane < NW ? sh.red[k][lane] : 0.0);
-      const double r = fabs(ref[k]);
-      E[k] = r > 0.0 && r < 1e300 ? (int)((__double_as_longlong(r) >> 52) & 2047) - 1023 + 40 : 40;
-      E[k] = max(-860, min(980, E[k]));
+      E[k] = sum_scale(ref[k]);
       res[k] = 0.0;
     }
     const bool mine = lane < 3 * NV;
@@ -1255,18 +1247,9 @@ __device__ bool grid_sum(GridSlots *S, SumShared &sh, int CS, int rank, SumState
       const int par = st.phase & 1;
       st.phase++;
       const double x = (NV > 1 && k0) ? t[NV - 1] : t[0];
-      const int e = (NV > 1 && k0) ? E[NV - 1] : E[0];
+      const int e = (NV > 1 && k0) ? E[NV - 1].e : E[0].e;
       unsigned long long *w = &S->w[(par * 6 + (mine ? lane : 0)) * kSumStride];
-      // this lane's limb: the mantissa of x shifted to the limb's lowest bit
-      // (bits below 2^(e - 130) are dropped), with the sign of x
-      const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
-      const int xe = (int)((xb >> 52) & 2047);
-      const int sft = xe - 1075 - (e - 38 - 46 * limb);
-      unsigned long long m = xe ? (xb & ((1ull << 52) - 1)) | (1ull << 52) : 0ull;
-      m = sft >= 0 ? (sft < 46 ? m << sft : 0ull) : (sft > -53 ? m >> -sft : 0ull);
-      if (limb > 0) m &= (1ull << 46) - 1;
-      long long add = (long long)xb < 0 ? -(long long)m : (long long)m;
-      if (xe - 1023 >= e) add = limb == 0 ? 1ll << 47 : 0;  // does not fit (or is not finite)
+      const long long add = sum_limb(x, e, limb);
       unsigned long long cur = 0;
       const unsigned long long seen = par ? st.seen[1] : st.seen[0];
       if (mine)
@@ -1287,20 +1270,13 @@ __device__ bool grid_sum(GridSlots *S, SumShared &sh, int CS, int rank, SumState
         if (par) st.seen[1] = cur; else st.seen[0] = cur;
       }
       again = false;
-      const double d = scale2((double)sum, e - 38 - 46 * (limb < 3 ? limb : 0));
+      const double d = scale2((double)sum, limb_exponent(e, limb));
 #pragma unroll
       for (int k = 0; k < NV; k++) {
-        const bool over = __shfl_sync(0xffffffffu, (int)(sum >= (1ll << 46)), 3 * k) != 0;
+        const bool over = __shfl_sync(0xffffffffu, (int)(sum >= kSumMarked), 3 * k) != 0;
         const double d1 = __shfl_sync(0xffffffffu, d, 3 * k + 1), d2 = __shfl_sync(0xffffffffu, d, 3 * k + 2);
         res[k] = __shfl_sync(0xffffffffu, d, 3 * k) + (d1 + d2);
-        const int re = (int)((__double_as_longlong(res[k]) >> 52) & 2047) - 1023;
-        if (over) {                                        // a partial did not fit
-          if (E[k] < 980) { E[k] = min(980, E[k] + 80); again = true; }
-          else res[k] = __longlong_as_double(0x7FF8000000000000ll);
-        } else if (re < E[k] - 66 && E[k] > -860) {        // fewer than 64 bits left
-          E[k] = max(-860, res[k] != 0.0 ? re + 20 : E[k] - 60);
-          again = true;
-        }
+        again = sum_again(E[k], over, res[k]) || again;
       }
       again = again && ok;
     }
