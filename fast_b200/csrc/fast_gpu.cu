@@ -181,6 +181,7 @@ int fast_gpu_create(int device, fast_gpu_ctx **out) {
   c->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->staged, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_status, sizeof(int32_t) * 4);
   if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_status, sizeof(int32_t) * 4);
@@ -306,6 +307,7 @@ int fast_gpu_destroy(fast_gpu_ctx *c) {
   if (c->h_state) cudaFreeHost(c->h_state);
   dfree(c->d_partials);
   if (c->d_bar) cudaFree(c->d_bar);
+  if (c->staged) cudaEventDestroy(c->staged);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   if (c->side_stream) cudaStreamDestroy(c->side_stream);
   delete c;
@@ -316,7 +318,10 @@ const char *fast_gpu_last_error(const fast_gpu_ctx *c) { return c ? c->err.c_str
 
 int fast_gpu_set_stream(fast_gpu_ctx *c, void *s) {
   if (check_ctx(c)) return FAST_GPU_EINVAL;
-  c->stream = s ? (cudaStream_t)s : c->own_stream;
+  cudaStream_t next = s ? (cudaStream_t)s : c->own_stream;
+  // (an event, not the old stream, which its owner may have destroyed)
+  if (next != c->stream) CK(cudaEventSynchronize(c->staged));
+  c->stream = next;
   return FAST_GPU_OK;
 }
 
@@ -587,6 +592,7 @@ int fast_gpu_update_coords(fast_gpu_ctx *c, const double *coords) {
     src = c->h_eq_tmp;
   }
   CK(cudaMemcpyAsync(c->d_X, src, sizeof(double) * 3 * c->nnode, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaEventRecord(c->staged, c->stream));
   c->mf.geo_ok = false;
   c->K_ok = c->M_ok = false;
   invalidate(*c, FAST_ASM_STIFFNESS);
@@ -622,6 +628,7 @@ int fast_gpu_update_material(fast_gpu_ctx *c, int32_t b, const double *E, const 
       gather_host(h, nu, B.perm.data(), B.ne);
       CK(cudaMemcpyAsync(B.d_nu, h, sizeof(double) * B.ne, cudaMemcpyHostToDevice, c->stream));
     }
+    CK(cudaEventRecord(c->staged, c->stream));
   }
   c->mf.mat_ok = false;
   c->K_ok = c->M_ok = false;
@@ -643,6 +650,7 @@ int fast_gpu_set_displacement(fast_gpu_ctx *c, const double *u) {
   copy_host(c->h_eq_tmp, u, nb);
   CK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp, nb, cudaMemcpyHostToDevice, c->stream));
   CK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_disp));
+  CK(cudaEventRecord(c->staged, c->stream));
   return FAST_GPU_OK;
 }
 

@@ -248,6 +248,9 @@ struct Ctx {
   PcgState *h_state = nullptr;    // pinned
   double *d_eq_tmp = nullptr;     // [neq] staging for host <-> device in equation space
   double *h_eq_tmp = nullptr;     // pinned [2 neq] staging: whoever fills it synchronises the stream first
+  // behind the last copy that an entry point left on its way from h_eq_tmp:
+  // a change of stream waits for it (the next fill synchronises the new stream only)
+  cudaEvent_t staged = nullptr;
 
   // matrix-free solves (matfree.cu)
   MatFree mf;
