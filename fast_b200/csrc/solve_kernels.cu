@@ -1930,12 +1930,20 @@ static bool use_persistent(Ctx &c) {
     sized(pcg_persistent<double, 16>);
     sized(pcg_persistent<float, 16>);
     sized(pcg_persistent<float, 8>);
-    if (!c.d_lcol && fits)
-      fits = cudaMalloc((void **)&c.d_lcol, sizeof(uint16_t) * std::max<int64_t>(4, c.nnzb_pad)) == cudaSuccess &&
-             cudaMalloc((void **)&c.d_z2, sizeof(double) * 4 * c.nnode) == cudaSuccess;
     if (!fits) {
       cudaGetLastError();
       c.persist_max_nodes = 0;
+      return false;
+    }
+    if ((!c.d_lcol &&
+         cudaMalloc((void **)&c.d_lcol, sizeof(uint16_t) * std::max<int64_t>(4, c.nnzb_pad)) != cudaSuccess) ||
+        (!c.d_z2 && cudaMalloc((void **)&c.d_z2, sizeof(double) * 4 * c.nnode) != cudaSuccess)) {
+      // no memory now: kernel by kernel this time, the next solve asks again
+      cudaFree(c.d_lcol);
+      cudaFree(c.d_z2);
+      c.d_lcol = nullptr;
+      c.d_z2 = nullptr;
+      cudaGetLastError();
       return false;
     }
     cudaGetLastError();

@@ -1,0 +1,52 @@
+"""What a call does where an allocation of device memory fails: the same
+result another way where one exists, and nothing half allocated is used
+afterwards."""
+import numpy as np
+import pytest
+
+from fast_b200 import decks, gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _box(kind, n, rho=None):
+    rng = np.random.default_rng(sum(n))
+    X, conn, _ = decks.box_mesh(kind, n, tuple(v / 8 for v in n))
+    X = X + rng.uniform(-0.04, 0.04, X.shape) / (16 if kind == "hex20" else 8)
+    fixed = np.zeros(X.shape, bool)
+    fixed[X[:, 2] < 0.02] = True
+    ne = len(conn)
+    g = 2 if kind == "hex8" else 3
+    d = decks.Deck(kind, X, conn, 1000.0 * np.exp(0.3 * rng.standard_normal(ne)), np.full(ne, 0.3), (g, g, g), fixed,
+                   matrix_type="sparse", rho=None if rho is None else np.full(ne, rho))
+    return d, rng.standard_normal(d.num_eq())
+
+
+# the persistent kernel's list indices (3.3 MB) and second z (2 MB): room for none, one, both
+@pytest.mark.parametrize("leave", [0, 4 << 20, 32 << 20])
+def test_persistent_kernel_buffers(leave):
+    from tests.device_memory import short_of_memory
+    d, f = _box("hex8", (39, 39, 38))
+    s = gpu.GpuSystem(0)
+    s.set_option(gpu.OPT_MATRIX_FREE, 10 ** 12)
+    s.upload(d)
+    s.assemble()
+    warm = gpu.GpuSystem(0)          # loads the kernels
+    warm.set_option(gpu.OPT_MATRIX_FREE, 10 ** 12)
+    warm.upload(d)
+    warm.assemble()
+    want, rep = warm.solve(f, tol=1e-10)
+    warm.close()
+    s.set_option(gpu.OPT_PERSISTENT_MAX_NODES, 0)
+    steps, _ = s.solve(f, tol=1e-10)
+    with short_of_memory(leave):
+        for _ in range(3):           # raising the limit again must not use half of the buffers
+            s.set_option(gpu.OPT_PERSISTENT_MAX_NODES, 65536)
+            u, r = s.solve(f, tol=1e-10)
+            assert r["converged"]
+            assert np.array_equal(u, steps) or np.array_equal(u, want)
+            if leave == 0:
+                assert np.array_equal(u, steps)
+    u, r = s.solve(f, tol=1e-10)     # memory is back: so is the kernel
+    assert np.array_equal(u, want) and r == rep
+    s.close()
