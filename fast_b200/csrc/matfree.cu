@@ -1229,12 +1229,16 @@ static cudaError_t solve_batch(Ctx &c, double tol, int maxit, bool warm, int32_t
     e = cudaSuccess;
     auto up = [&](auto **p, const auto &v) {
       if (e == cudaSuccess && !*p) e = cudaMalloc((void **)p, sizeof(v[0]) * std::max<size_t>(1, v.size()));
-      if (e == cudaSuccess) e = cudaMemcpy(*p, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(*p, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice, c.stream);
     };
     up(&M.bprob, bp);
     up(&M.ntile, nt);
     up(&M.eptr, M.h_eptr);
     up(&M.nptr, M.h_ntile);
+    // (on the solve's own stream, which the legacy stream does not order, and done before bp and nt go)
+    const cudaError_t es = cudaStreamSynchronize(c.stream);
+    if (e == cudaSuccess) e = es;
     if (e == cudaSuccess && !M.bpart) e = cudaMalloc((void **)&M.bpart, sizeof(double) * (M.nb + 2 * nt.size() + 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&M.S, sizeof(MfProblem) * np);
     if (e != cudaSuccess) return e;

@@ -55,3 +55,39 @@ def test_stream_changes_between_calls(n):
     many.assemble()
     one.close()
     many.close()
+
+
+def test_first_batched_solve_on_a_callers_stream():
+    """The tables of an ensemble's first solve are uploaded on the stream that
+    reads them: the first solve of a fresh context gives the second one's bits."""
+    import torch
+    off = [0]
+    rng = np.random.default_rng(3)
+    Xs, cs, fs = [], [], []
+    for n in [(3 + k % 5, 3 + k % 3, 2 + k % 4) for k in range(64)]:
+        X, conn, _ = decks.box_mesh("hex8", n, (1.0, 1.0, 1.0))
+        fixed = np.zeros(X.shape, bool)
+        fixed[X[:, 0] < 1e-9] = True
+        Xs.append(X)
+        cs.append(conn + off[-1])
+        fs.append(fixed)
+        off.append(off[-1] + len(X))
+    conn = np.concatenate(cs)
+    ne = len(conn)
+    d = decks.Deck("hex8", np.concatenate(Xs), conn, 1000.0 * np.exp(0.3 * rng.standard_normal(ne)),
+                   np.full(ne, 0.3), (2, 2, 2), np.concatenate(fs), matrix_type="sparse")
+    f = rng.standard_normal(d.num_eq())
+    first = None
+    for k in range(8):
+        stream = torch.cuda.Stream()
+        s = gpu.GpuSystem(0)
+        s.set_stream(stream.cuda_stream)
+        s.set_option(gpu.OPT_MATRIX_FREE, 0)
+        s.upload(d)
+        s.set_problems(np.asarray(off))
+        s.assemble()
+        u = s.solve_batch(f, tol=1e-10)[0]
+        assert np.array_equal(u, s.solve_batch(f, tol=1e-10)[0])
+        first = u if first is None else first
+        assert np.array_equal(u, first)
+        s.close()
