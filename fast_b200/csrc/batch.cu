@@ -104,9 +104,15 @@ extern "C" int fast_gpu_solve_batch(fast_gpu_ctx *c, const double *f, double *u,
   for (int k = 0; k < c->nprob; k++) biggest = std::max(biggest, c->h_noff[k + 1] - c->h_noff[k]);
   const int maxit = opts.maxit > 0 ? opts.maxit : (int)std::max<int64_t>(60 * biggest, 100);
   if (c->precond_built != opts.precond) BCK(launch_build_precond(*c, c->d_K, opts.precond));
-  const bool mf = mf_batch_active(*c);
-  if (mf) BCK(mf_prepare(*c, false, opts.precond));
-  else BCK(solve_layout(*c, FAST_ASM_STIFFNESS, false));
+  // matrix-free where its operands find memory
+  bool mf = mf_batch_active(*c);
+  auto found_memory = [&](cudaError_t e) -> cudaError_t {
+    if (e != cudaErrorMemoryAllocation) return e;
+    mf_give_up(*c);
+    mf = false;
+    return cudaSuccess;
+  };
+  if (mf) BCK(found_memory(mf_prepare(*c, false, opts.precond)));
   const size_t nb = sizeof(double) * c->neq;
   BCK(cudaStreamSynchronize(c->stream));
   copy_host(c->h_eq_tmp, f, nb);
@@ -121,9 +127,9 @@ extern "C" int fast_gpu_solve_batch(fast_gpu_ctx *c, const double *f, double *u,
   std::vector<int32_t> it(c->nprob), dn(c->nprob);
   std::vector<double> er(c->nprob);
   const int64_t sp = c->begin_span(FAST_KERNEL_LINEAR_SOLVE);
-  if (mf) {
-    BCK(mf_solve_batch(*c, tol, maxit, warm, it.data(), er.data(), dn.data()));
-  } else {
+  if (mf) BCK(found_memory(mf_solve_batch(*c, tol, maxit, warm, it.data(), er.data(), dn.data())));
+  if (!mf) {
+    BCK(solve_layout(*c, FAST_ASM_STIFFNESS, false));
     BCK(launch_pcg_batch(*c, c->nprob, c->d_order, c->d_noff, tol, maxit, warm, c->d_piters, c->d_perr, c->d_pdone));
     BCK(cudaMemcpyAsync(it.data(), c->d_piters, sizeof(int32_t) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
     BCK(cudaMemcpyAsync(dn.data(), c->d_pdone, sizeof(int32_t) * c->nprob, cudaMemcpyDeviceToHost, c->stream));

@@ -850,10 +850,22 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
   if (c->precond_built != precond)
     CK(k32 ? launch_build_precond32(*c, c->d_K32, precond) : launch_build_precond(*c, c->d_K, precond));
   c->mf_fp32 = mixed;
-  const bool mf = mf_active(*c);
+  bool mf = mf_active(*c);
+  // without memory for its operands this solve goes to the assembled matrix, whose layout may be there
+  const OnAssembledMatrix restore(*c);
+  c->mf_off = restore.was;
+  if (mf) {
+    const cudaError_t e = mf_prepare(*c, mixed, precond);
+    if (e == cudaErrorMemoryAllocation) {
+      mf_give_up(*c);
+      mf = false;
+      c->mf_off = true;
+    } else {
+      CK(e);
+    }
+  }
   c->mf_used = mf;
   if (mf) {
-    CK(mf_prepare(*c, mixed, precond));
     if (c->graph_mf_precond != precond) c->drop_graphs();
     c->graph_mf_precond = precond;
   } else {

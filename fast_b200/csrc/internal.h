@@ -327,10 +327,13 @@ struct Ctx {
   cudaGraphExec_t graph_mf64 = nullptr, graph_mf32 = nullptr;
   int graph_mf64_chunk = 0, graph_mf32_chunk = 0, graph_mf_precond = -1;
   int64_t graph_mf64_kernels = 0, graph_mf32_kernels = 0;
-  void drop_graphs() {
+  void drop_mf_graphs() {
     if (graph_mf64) cudaGraphExecDestroy(graph_mf64);
     if (graph_mf32) cudaGraphExecDestroy(graph_mf32);
     graph_mf64 = graph_mf32 = nullptr;
+  }
+  void drop_graphs() {
+    drop_mf_graphs();
     if (graph_fp64) cudaGraphExecDestroy(graph_fp64);
     if (graph_mixed) cudaGraphExecDestroy(graph_mixed);
     graph_fp64 = graph_mixed = nullptr;
@@ -487,6 +490,8 @@ cudaError_t launch_to_soa(Ctx &c, const double *K, double *Ks, float *Ks32);
 // *skip
 bool mf_active(const Ctx &c);
 cudaError_t mf_prepare(Ctx &c, bool fp32, int precond);
+// after cudaErrorMemoryAllocation: what it has is given back
+void mf_give_up(Ctx &c);
 template <typename T>
 void mf_iterations(Ctx &c, int k, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr);
 cudaError_t mf_residual_of(Ctx &c, const double *f, const double *u, double *r, double *part, int nparts,

@@ -1173,6 +1173,13 @@ cudaError_t mf_prepare(Ctx &c, bool fp32, int precond) {
   }
 }
 
+void mf_give_up(Ctx &c) {
+  (void)cudaGetLastError();
+  cudaStreamSynchronize(c.stream);
+  c.drop_mf_graphs();
+  c.mf.release();
+}
+
 template <typename T>
 void mf_iterations(Ctx &c, int k, T *u, T *r, T *z, T *p, double *part_pw, double *part_rr, double *part_zr) {
   const MatFree &M = c.mf;

@@ -1971,7 +1971,7 @@ static cudaError_t drive(Ctx &c, int maxit, int chunk, cudaGraphExec_t *graph, i
   cudaError_t e;
   cudaEvent_t ev;
   if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
-  const bool use_graph = graph != nullptr && !c.timing;
+  bool use_graph = graph != nullptr && !c.timing;
   int launched = 0;
   bool pending = false;
   while (true) {
@@ -1988,10 +1988,17 @@ static cudaError_t drive(Ctx &c, int maxit, int chunk, cudaGraphExec_t *graph, i
         if (el != cudaSuccess) e = el;
         if (e == cudaSuccess) e = cudaGraphInstantiate(graph, g, 0);
         if (g) cudaGraphDestroy(g);
+        const int64_t kernels = c.launches - before;
+        c.launches = before;
+        if (e == cudaErrorMemoryAllocation) {  // no room for a graph: without it
+          *graph = nullptr;
+          (void)cudaGetLastError();
+          use_graph = false;
+          continue;
+        }
         if (e != cudaSuccess) { *graph = nullptr; break; }
         *graph_chunk = chunk;
-        *graph_kernels = c.launches - before;
-        c.launches = before;
+        *graph_kernels = kernels;
       }
       if ((e = cudaGraphLaunch(*graph, c.stream)) != cudaSuccess) break;
       c.launches += *graph_kernels;

@@ -50,3 +50,60 @@ def test_persistent_kernel_buffers(leave):
     u, r = s.solve(f, tol=1e-10)     # memory is back: so is the kernel
     assert np.array_equal(u, want) and r == rep
     s.close()
+
+
+@pytest.mark.parametrize("precision", [gpu.PREC_FP64, gpu.PREC_MIXED])
+def test_matrix_free_solve_falls_back(precision):
+    """No memory for the matrix-free operands: the assembled matrix, whose
+    layout is there, solves; matrix-free again once there is memory."""
+    from tests.device_memory import short_of_memory
+    d, f = _box("hex20", (14, 13, 12))
+    s = gpu.GpuSystem(0)
+    s.upload(d)
+    s.set_option(gpu.OPT_PERSISTENT_MAX_NODES, 0)
+    s.assemble()
+
+    def solve():
+        before = s.launch_count()
+        u, r = s.solve(f, tol=1e-10, precision=precision)
+        return u, r, (s.launch_count() - before) / r["iterations"]
+
+    s.set_option(gpu.OPT_MATRIX_FREE, 0)
+    free, rf, per_free = solve()
+    assert per_free < 3.0
+    s.set_option(gpu.OPT_MATRIX_FREE, 10 ** 12)
+    asm, ra, per_asm = solve()
+    assert per_asm >= 3.0
+    s.upload(d)                        # the operands go, the layouts too
+    s.assemble()
+    assert np.array_equal(solve()[0], asm)
+    s.set_option(gpu.OPT_MATRIX_FREE, 0)
+    for leave in (0, 12 << 20):        # 2,184 elements: 4 MB of geometry, 2 MB of element forces
+        with short_of_memory(leave):
+            u, r, per = solve()
+            assert np.array_equal(u, asm) or np.array_equal(u, free)
+            if leave == 0:
+                assert np.array_equal(u, asm) and r == ra and per >= 3.0
+    u, r, per = solve()
+    assert np.array_equal(u, free) and r == rf
+    s.close()
+
+
+def test_ensemble_falls_back():
+    from tests.device_memory import short_of_memory
+    from tests.test_gpu_batch_lockstep import _members
+    d, off, f = _members([(10, 9, 8)] * 40)
+    s = gpu.GpuSystem(0)
+    s.upload(d)
+    s.set_problems(off)
+    s.assemble()
+    s.set_option(gpu.OPT_MATRIX_FREE, 0)
+    free = s.solve_batch(f, tol=1e-10)[0]
+    s.set_option(gpu.OPT_MATRIX_FREE, 10 ** 12)
+    asm = s.solve_batch(f, tol=1e-10)[0]
+    s.set_problems(off)                # the operands go, the layout stays
+    s.set_option(gpu.OPT_MATRIX_FREE, 0)
+    with short_of_memory():
+        assert np.array_equal(s.solve_batch(f, tol=1e-10)[0], asm)
+    assert np.array_equal(s.solve_batch(f, tol=1e-10)[0], free)
+    s.close()
