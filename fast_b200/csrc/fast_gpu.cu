@@ -744,6 +744,7 @@ int fast_gpu_assemble(fast_gpu_ctx *c, int32_t what) {
   CK(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->harvest();
+  if (what == FAST_ASM_MASS) mass_rows_done(*c);
   if (what == FAST_ASM_STIFFNESS) c->K_ok = true; else c->M_ok = true;
   invalidate(*c, what);
   if (c->h_status[0] & 1) {

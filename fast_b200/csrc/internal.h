@@ -439,6 +439,7 @@ cudaError_t launch_element_matrices(Ctx &c, int what, int bucket, int64_t first_
 // mass_rows.cu: every block of M stored (no zero fill); cudaErrorNotSupported
 // where launch_assemble has to add it
 cudaError_t launch_mass_rows(Ctx &c, double *M);
+void mass_rows_done(Ctx &c);  // when the stream is
 // geom.cu: G += sign * geometric stiffness at c.d_disp (small-strain hex
 // buckets, colour by colour; fixed rows and columns untouched)
 cudaError_t launch_geom_stiffness(Ctx &c, double *G, double sign);

@@ -181,4 +181,18 @@ cudaError_t launch_mass_rows(Ctx &c, double *M) {
   return B.nn == 8 ? go<8>(c, B, M) : go<20>(c, B, M);
 }
 
+// The pair numbers are kept for the next assembly up to 1 GB (335,544 hex20
+// elements); a larger array is given back once the stream is done with it, so
+// that the solve's layouts find room.  Making it anew costs as much as the
+// assembly: 11.0 ms an assembly of 648,000 elements (2.1 GB), 5.3 if it is kept,
+// 19.6 by the coloured scatter; at 131,072 (420 MB) 2.1, 1.1 and 4.0.
+void mass_rows_done(Ctx &c) {
+  constexpr size_t kKeep = (size_t)1 << 30;
+  if (!c.d_mpairs) return;
+  const Bucket &B = c.buckets[0];
+  if (sizeof(double) * (size_t)B.ne * B.nn * B.nn <= kKeep) return;
+  cudaFree(c.d_mpairs);
+  c.d_mpairs = nullptr;
+}
+
 }  // namespace fastgpu

@@ -107,3 +107,38 @@ def test_ensemble_falls_back():
         assert np.array_equal(s.solve_batch(f, tol=1e-10)[0], asm)
     assert np.array_equal(s.solve_batch(f, tol=1e-10)[0], free)
     s.close()
+
+
+@pytest.mark.parametrize("n,kept", [((24, 24, 24), True), ((70, 70, 69), False)])   # 44 MB and 1.08 GB of pair numbers
+def test_mass_assembly_keeps_little(n, kept):
+    """A large array of mass numbers per node pair is given back; the next
+    assembly gives the same bits, and without room for it the element-wise
+    scatter takes its place."""
+    import torch
+    from tests.device_memory import short_of_memory
+    d, f = _box("hex20", n, rho=1e-3)
+    x = np.random.default_rng(1).standard_normal(d.num_eq())
+    s = gpu.GpuSystem(0)
+    s.upload(d)
+    s.assemble()
+    s.assemble_mass()                     # M itself is there from here on
+    y = s.mult_vect(x, gpu.ASM_M)
+    s.upload(d)
+    s.assemble()
+    s._ck(s.L.fast_gpu_zero(s.ctx, gpu.ASM_M), "zero")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    s.assemble_mass()
+    torch.cuda.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    size = 8 * 400 * n[0] * n[1] * n[2]
+    assert used >= size if kept else used < 4 << 20
+    assert np.array_equal(s.mult_vect(x, gpu.ASM_M), y)
+    s.assemble_mass()
+    assert np.array_equal(s.mult_vect(x, gpu.ASM_M), y)
+    if not kept:
+        with short_of_memory():
+            s.assemble_mass()
+        z = s.mult_vect(x, gpu.ASM_M)
+        assert np.abs(z - y).max() <= 1e-13 * np.abs(y).max()   # another order of at most 8 sums a block, 81 blocks a row
+    s.close()
