@@ -97,6 +97,7 @@ double *target_of(Ctx &c, int what) {
 }
 
 void invalidate(Ctx &c, int what) {
+  c.products[what == FAST_ASM_MASS] = 0;
   if (what == FAST_ASM_STIFFNESS) { c.Ks_ok = false; c.precond_built = -1; c.K_pure = false; }
   else c.Ms_ok = false;
 }
@@ -817,9 +818,17 @@ int fast_gpu_mult_vect(fast_gpu_ctx *c, int32_t what, const double *x, double *y
   copy_host(c->h_eq_tmp, x, nb);
   CK(cudaMemcpyAsync(c->d_eq_tmp, c->h_eq_tmp, nb, cudaMemcpyHostToDevice, c->stream));
   CK(launch_eq_to_node(*c, c->d_eq_tmp, c->d_z));
-  // the solve layout where it is there: a product takes 112 us on it and 127 on
-  // the blocks (32,760 hex20 elements), but making it 240
-  if (what == FAST_ASM_MASS ? c->Ms_ok : c->Ks_ok)
+  // the solve layout where it is there: a product takes 103 us on it and 125 on
+  // the blocks (32,760 hex20 elements; 120,000 hex8: 54 and 64), but making it
+  // 240 (117); so it is made after 12 products with the same matrix, if it finds
+  // memory.  The bits are the same.
+  const bool &there = what == FAST_ASM_MASS ? c->Ms_ok : c->Ks_ok;
+  if (!there && ++c->products[what == FAST_ASM_MASS] > 12) {
+    const cudaError_t e = ensure_soa(*c, what, false);
+    if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+    else CK(e);
+  }
+  if (there)
     CK(launch_spmv(*c, what == FAST_ASM_MASS ? c->d_Ms : c->d_Ks, c->d_z, c->d_w));
   else
     CK(launch_spmv_blocks(*c, T, c->d_z, c->d_w));

@@ -979,43 +979,84 @@ cudaError_t launch_matfree_residual(Ctx &c, const double *f, const double *u, do
 }
 
 // y = K x from the 3x3 blocks as assembled, row-major, for a product or two of a
-// matrix that no solve has asked a layout for.  A warp per block-row; 27 lanes
-// take three whole blocks (216 bytes) at a time, each lane one entry of a
-// block, so loads are whole lines and a lane's row and column never change.
-// 563 MB in 127 us, where the solve layout's product takes 112 and making that
-// layout 240.  (Eight trips of three blocks in flight and a grid of eight blocks
-// per SM, of which five fit, took 158; six blocks per SM, with spills, 224.)
-__global__ void __launch_bounds__(kSpmvThreads, 5)
+// matrix that no solve has asked a layout for.  Lanes per row, blocks per lane
+// and order of sums are spmv_f64's: the same bits whichever runs.  A warp copies
+// the next 64 blocks of its rows to shared memory, consecutive lanes taking
+// consecutive entries (a lane reading its own two blocks, 144 bytes from the
+// next lane's, would touch a line per lane and entry), and each lane takes its
+// blocks from there.  Measured on 32,760 hex20 / 120,000 hex8 elements (563 /
+// 243 MB): 125 / 64 us, where the solve layout's product takes 103 / 54 and
+// making that layout 240 / 117.  (27 lanes taking three whole blocks at a time
+// from memory, another order of sums: 133 / 69; through registers instead of
+// cp.async, 5 blocks per SM and spills: 216 / 102.)
+template <int LPR>
+__global__ void __launch_bounds__(kSpmvThreads, 4)
 spmv_blocks(int64_t nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
             const double *__restrict__ K, const double *__restrict__ x, double *__restrict__ y) {
-  const int lane = threadIdx.x & 31, kb = lane / 9, k = lane - 9 * kb, j = k % 3;
-  constexpr int U = 7;  // 21 blocks in flight: hex20 rows of 51, 57 and 81, hex8 ones of 27
-  for (int64_t n = (blockIdx.x * (int64_t)kSpmvThreads + threadIdx.x) >> 5; n < nrows;
-       n += ((int64_t)gridDim.x * kSpmvThreads) >> 5) {
-    const int32_t b0 = rowptr[n], b1 = rowptr[n + 1];
-    double s = 0.0;
-    for (int32_t b = b0; b < b1; b += 3 * U) {
-      double v[U], xv[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int32_t at = b + 3 * u + kb;
-        const bool in = kb < 3 && at < b1;
-        v[u] = in ? K[9 * (int64_t)at + k] : 0.0;
-        xv[u] = in ? x[4 * (int64_t)col[at] + j] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) s += v[u] * xv[u];
+  constexpr int RPW = 32 / LPR, N = 18 * LPR;  // rows of a warp, entries of a row's trip
+  __shared__ double sv[kSpmvThreads / 32][19 * 32];  // (19: the lanes' blocks start on different banks)
+  const int lane = threadIdx.x & 31, q = lane % LPR;
+  const unsigned w = (unsigned)__cvta_generic_to_shared(sv[threadIdx.x >> 5]);
+  const double *v = sv[threadIdx.x >> 5] + 19 * lane;
+  const int64_t warp = (blockIdx.x * (int64_t)kSpmvThreads + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * kSpmvThreads) >> 5;
+  for (int64_t row0 = warp * RPW; row0 < nrows; row0 += nwarps * RPW) {
+    const int64_t row = row0 + lane / LPR;
+    const bool live = row < nrows;
+    int32_t b0 = 0, nb = 0;
+    if (live) {
+      b0 = rowptr[row];
+      nb = rowptr[row + 1] - b0;
     }
-    // lanes 9 kb + 3 i + j -> row i
-    s += __shfl_down_sync(0xffffffffu, s, 9) + __shfl_down_sync(0xffffffffu, s, 18);
-    s += __shfl_down_sync(0xffffffffu, s, 1) + __shfl_down_sync(0xffffffffu, s, 2);
-    const double s1 = __shfl_down_sync(0xffffffffu, s, 3), s2 = __shfl_down_sync(0xffffffffu, s, 6);
-    if (lane == 0) V4<double>::store(y + 4 * n, s, s1, s2);
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    const int32_t most = __reduce_max_sync(0xffffffffu, nb);
+    for (int32_t j0 = 0; j0 < most; j0 += 2 * LPR) {
+      const int32_t j = j0 + 2 * q;
+#pragma unroll
+      for (int r = 0; r < RPW; r++) {
+        const double *g = K + 9 * (int64_t)__shfl_sync(0xffffffffu, b0 + j0, r * LPR);
+        const int32_t n = min(N, 9 * __shfl_sync(0xffffffffu, nb - j0, r * LPR));
+#pragma unroll
+        for (int i = 0; i < (N + 31) / 32; i++) {
+          const int e = 32 * i + lane;
+          if (e < n)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(w + 8 * (r * 19 * LPR + e + e / 18)), "l"(g + e)
+                         : "memory");
+        }
+      }
+      double xa0 = 0, xa1 = 0, xa2 = 0, xb0 = 0, xb1 = 0, xb2 = 0;
+      if (j < nb) V4<double>::load(x + 4 * (int64_t)col[b0 + j], xa0, xa1, xa2);
+      if (j + 1 < nb) V4<double>::load(x + 4 * (int64_t)col[b0 + j + 1], xb0, xb1, xb2);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      if (j < nb) {
+        double o[9];
+#pragma unroll
+        for (int i = 0; i < 9; i++) o[i] = j + 1 < nb ? v[9 + i] : 0.0;
+        a0 += v[0] * xa0 + v[1] * xa1 + v[2] * xa2 + o[0] * xb0 + o[1] * xb1 + o[2] * xb2;
+        a1 += v[3] * xa0 + v[4] * xa1 + v[5] * xa2 + o[3] * xb0 + o[4] * xb1 + o[5] * xb2;
+        a2 += v[6] * xa0 + v[7] * xa1 + v[8] * xa2 + o[6] * xb0 + o[7] * xb1 + o[8] * xb2;
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) {
+      a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+      a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+      a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+    if (live && q == 0) V4<double>::store(y + 4 * row, a0, a1, a2);
   }
 }
 
 cudaError_t launch_spmv_blocks(Ctx &c, const double *K, const double *x, double *y) {
-  spmv_blocks<<<5 * c.sm_count, kSpmvThreads, 0, c.stream>>>(c.nnode, c.d_rowptr, c.d_col, K, x, y);
+  const int G = 4 * c.sm_count;
+  switch (c.lpr64) {
+    case 4: spmv_blocks<4><<<G, kSpmvThreads, 0, c.stream>>>(c.nnode, c.d_rowptr, c.d_col, K, x, y); break;
+    case 8: spmv_blocks<8><<<G, kSpmvThreads, 0, c.stream>>>(c.nnode, c.d_rowptr, c.d_col, K, x, y); break;
+    case 32: spmv_blocks<32><<<G, kSpmvThreads, 0, c.stream>>>(c.nnode, c.d_rowptr, c.d_col, K, x, y); break;
+    default: spmv_blocks<16><<<G, kSpmvThreads, 0, c.stream>>>(c.nnode, c.d_rowptr, c.d_col, K, x, y);
+  }
   c.launches++;
   return cudaGetLastError();
 }
