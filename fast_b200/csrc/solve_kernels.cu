@@ -2116,8 +2116,10 @@ static void mixed_init(Ctx &c, bool warm, double tol, const double *tol_dev, int
   if (!warm) cudaMemsetAsync(c.d_u, 0, sizeof(double) * 4 * nn, c.stream);
   cudaMemsetAsync(c.s_x, 0, sizeof(float) * 4 * nn, c.stream);
   sumsq_kernel<<<R, 256, 0, c.stream>>>(4 * nn, c.d_f, P_D(c));
-  // the tensor-core stiffness may restart its recurrence (see reliable_scalar)
-  mixed_init_scalar<<<1, 256, 0, c.stream>>>(c.d_state, P_D(c), R, tol, tol_dev, maxit, c.K32_current ? 40 : 0);
+  // the tensor-core stiffness may restart its recurrence (see reliable_scalar);
+  // the matrix-free operator is the same in both precisions
+  mixed_init_scalar<<<1, 256, 0, c.stream>>>(c.d_state, P_D(c), R, tol, tol_dev, maxit,
+                                             c.K32_current && !mf_active(c) ? 40 : 0);
   c.launches += 2;
 }
 

@@ -1,0 +1,40 @@
+"""How long a mixed solve waits for FP32 before FP64 takes over
+(reliable_scalar): FP64 residuals formed (`outer`) in models where CG's residual
+does not halve for hundreds of iterations."""
+import numpy as np
+import pytest
+
+from fast_b200 import decks, gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(kind, n, L, sigma=0.5, seed=11):
+    rng = np.random.default_rng(seed)
+    X, conn, _ = decks.box_mesh(kind, n, L)
+    h = np.asarray(L) / np.asarray(n) / (2 if kind == "hex20" else 1)
+    Y = X + rng.uniform(-0.05, 0.05, X.shape) * h
+    fixed = np.zeros(X.shape, bool)
+    fixed[np.abs(X[:, 0]) < 1e-9] = True
+    ne = len(conn)
+    g = 2 if kind == "hex8" else 3
+    d = decks.Deck(kind, Y, conn, 1000.0 * np.exp(sigma * rng.standard_normal(ne)), np.full(ne, 0.3), (g, g, g),
+                   fixed, matrix_type="sparse")
+    f = np.zeros(d.num_eq())
+    q = d.node_eq()[np.abs(X[:, 0] - L[0]) < 1e-9, 2]
+    f[q[q > 0] - 1] = -1.0 / len(q)
+    return d, f
+
+
+def test_no_restarts_on_the_matrix_free_operator():
+    """After tensor-core assembly the assembled FP32 matrix may restart its
+    recurrence 40 times before it gives up (each after 10 residuals at the
+    least); the matrix-free operator is the FP64 one rounded, and does not."""
+    d, f = _model("hex20", (100, 5, 5), (100.0, 5.0, 5.0))
+    s = gpu.GpuSystem(0)
+    s.set_option(gpu.OPT_MATRIX_FREE, 0)
+    s.upload(d)
+    s.assemble(gpu.ASM_K_TF32)
+    u, rep = s.solve(f, tol=1e-8, precision=gpu.PREC_MIXED)
+    assert rep["converged"] and rep["escalated"] == 1 and rep["outer"] < 400
+    s.close()
