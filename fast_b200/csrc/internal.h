@@ -43,7 +43,7 @@ struct PcgState {
   int32_t restarts_left;    // mixed path: fresh starts of the recurrence still allowed after a stall
   int32_t fresh;            // the last FP64 residual restarts the recurrence (p = z)
   int32_t restarts;         // fresh starts taken
-  int32_t pad_;
+  int32_t plateau;          // mixed path: replacements without a 2x improvement while both residuals agree
 };
 
 // 32-bit words of one element's first-touch flags: nn*nn bits, rows padded

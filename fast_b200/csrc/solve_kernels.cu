@@ -621,10 +621,9 @@ __global__ void __launch_bounds__(256) reliable_scalar(PcgState *st, const doubl
     // The FP64 residual must halve within 10 replacements (10 chunks of FP32
     // iterations) and must not grow 100x above its best; otherwise FP32
     // iterates cannot resolve this system (cond(K) * eps_fp32 near 1).  While
-    // the recurrence's residual still is the true one (to 1 %), FP32 does
-    // resolve it and the plateau is CG's own: 40 replacements then (a 1.6
-    // million equation box shows plateaus of 650 iterations; giving up on them
-    // cost it 1,500 FP64 iterations, 458 against 308 ms).  Where
+    // the recurrence's residual still is the true one (to 1 %), FP32 may well
+    // resolve it and the plateau be CG's own: `plateau` replacements then
+    // (kPlateau).  Where
     // the FP32 operator is not the rounded FP64 one (the tensor-core
     // stiffness against the element-by-element FP64 residual) the search
     // directions stop fitting the replaced residuals first: the recurrence
@@ -635,7 +634,7 @@ __global__ void __launch_bounds__(256) reliable_scalar(PcgState *st, const doubl
     if (!grew && (st->updates == 1 || st->err_true < 0.5 * st->best_err)) {
       st->best_err = st->err_true;
       st->stall = 0;
-    } else if (grew || ++st->stall >= (fabs(st->err_true - err_rec) < 0.01 * st->err_true ? 40 : 10)) {
+    } else if (grew || ++st->stall >= (fabs(st->err_true - err_rec) < 0.01 * st->err_true ? st->plateau : 10)) {
       if (st->restarts_left <= 0) { st->done = 4; return; }
       st->restarts_left--;
       st->restarts++;
@@ -666,7 +665,8 @@ __global__ void keep_best(int64_t n4, const double *__restrict__ u, double *__re
 
 // mixed path start: lenf = |f| (with the reference's normaliser)
 __global__ void __launch_bounds__(256) mixed_init_scalar(PcgState *st, const double *part_ff, int nf, double tol,
-                                                         const double *tol_dev, int maxit, int restarts) {
+                                                         const double *tol_dev, int maxit, int restarts,
+                                                         int plateau) {
   if (tol_dev) tol = *tol_dev;
   __shared__ double sbuf[32];
   const double ff = sum_partials(part_ff, nf, sbuf);
@@ -676,6 +676,7 @@ __global__ void __launch_bounds__(256) mixed_init_scalar(PcgState *st, const dou
     s.tol = tol;
     s.maxit = maxit;
     s.restarts_left = restarts;
+    s.plateau = plateau;
     if (lenf < tol) { s.done = 1; s.null_rhs = 1; }   // PCGSolver returns at once for a null load
     if (lenf > 10e+10) lenf = 1.0;
     s.lenf = lenf > 0.0 ? lenf : 1.0;
@@ -2110,7 +2111,19 @@ static void fp64_chunk(Ctx &c, int k) {
   }
 }
 
-static void mixed_init(Ctx &c, bool warm, double tol, const double *tol_dev, int maxit) {
+// How many replacements a plateau of CG may last (reliable_scalar) before FP64
+// takes over.  Giving up early costs what FP32 saves over FP64, waiting in vain
+// 50 FP32 iterations a replacement.  Kernel by kernel or matrix-free an FP64
+// iteration takes 1.7 times an FP32 one.  Limit 10 / 40, ms: hex20 64x64x32,
+// four of six draws 335-373 / 240-260; hex8 60x60x60 with moduli over e^(+-4),
+// four draws 185-245 / 104-175; where FP32 fails all the same, hex20 30x30x30
+// with such moduli, 220-295 / 233-302.  In the persistent kernel the two
+// precisions are close and none of nine slender or nearly incompressible models
+// gained: 61 / 69, 70 / 82, 86 / 96, 59 / 64.  A recorded solve, which has no
+// FP64 iteration to go to, waits.
+constexpr int kPlateau = 40, kPlateauPersistent = 10;
+
+static void mixed_init(Ctx &c, bool warm, double tol, const double *tol_dev, int maxit, int plateau) {
   const int64_t nn = c.nnode;
   const int R = kRedBlocks;
   if (!warm) cudaMemsetAsync(c.d_u, 0, sizeof(double) * 4 * nn, c.stream);
@@ -2119,7 +2132,7 @@ static void mixed_init(Ctx &c, bool warm, double tol, const double *tol_dev, int
   // the tensor-core stiffness may restart its recurrence (see reliable_scalar);
   // the matrix-free operator is the same in both precisions
   mixed_init_scalar<<<1, 256, 0, c.stream>>>(c.d_state, P_D(c), R, tol, tol_dev, maxit,
-                                             c.K32_current && !mf_active(c) ? 40 : 0);
+                                             c.K32_current && !mf_active(c) ? 40 : 0, plateau);
   c.launches += 2;
 }
 
@@ -2201,7 +2214,7 @@ cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int it
 // FP32 PCG with FP64 reliable updates every `chunk` iterations.
 cudaError_t pcg_mixed(Ctx &c, bool warm, double tol, int maxit, int chunk) {
   cudaError_t e;
-  mixed_init(c, warm, tol, nullptr, maxit);
+  mixed_init(c, warm, tol, nullptr, maxit, !mf_active(c) && use_persistent(c) ? kPlateauPersistent : kPlateau);
   mixed_reliable(c);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (mf_active(c))
@@ -2233,7 +2246,7 @@ __global__ void pcg_loop_cond(cudaGraphConditionalHandle h, const PcgState *__re
 cudaError_t record_pcg(Ctx &c, bool mixed, bool warm, double tol, const double *tol_dev, int maxit, int chunk) {
   cudaError_t e;
   if (mixed) {
-    mixed_init(c, warm, tol, tol_dev, maxit);
+    mixed_init(c, warm, tol, tol_dev, maxit, kPlateau);
     mixed_reliable(c);
   } else {
     fp64_init(c, warm, tol, tol_dev, maxit, 0);

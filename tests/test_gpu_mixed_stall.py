@@ -38,3 +38,30 @@ def test_no_restarts_on_the_matrix_free_operator():
     u, rep = s.solve(f, tol=1e-8, precision=gpu.PREC_MIXED)
     assert rep["converged"] and rep["escalated"] == 1 and rep["outer"] < 400
     s.close()
+
+
+@pytest.mark.parametrize("kind,n,L", [("hex8", (200, 2, 2), (200.0, 2.0, 2.0)), ("hex20", (60, 3, 3), (60.0, 3.0, 3.0)),
+                                      ("hex8", (60, 60, 1), (60.0, 60.0, 0.5))])
+def test_persistent_kernel_gives_up_after_ten(kind, n, L):
+    """The first residual and ten without a halving."""
+    d, f = _model(kind, n, L)
+    s = gpu.GpuSystem(0)
+    s.upload(d)
+    s.assemble()
+    u, rep = s.solve(f, tol=1e-8, precision=gpu.PREC_MIXED)
+    assert rep["converged"] and rep["escalated"] == 1 and rep["outer"] == 11
+    s.close()
+
+
+@pytest.mark.parametrize("least", [0, 10 ** 12])
+def test_large_system_waits_out_a_plateau(least):
+    """On a large system (matrix-free or kernel by kernel) a plateau of ten
+    residuals is no reason to give up."""
+    d, f = _model("hex8", (60, 60, 60), (1.0, 1.0, 1.0), sigma=2.0)
+    s = gpu.GpuSystem(0)
+    s.set_option(gpu.OPT_MATRIX_FREE, least)
+    s.upload(d)
+    s.assemble()
+    u, rep = s.solve(f, tol=1e-8, precision=gpu.PREC_MIXED)
+    assert rep["converged"] and rep["escalated"] == 0 and rep["outer"] > 11
+    s.close()
