@@ -279,6 +279,12 @@ static int subspace_iteration(fast_gpu_ctx *c, const fast_gpu_modal_opts *o, boo
   // (a square root): with it the hex20 buckling column wandered around the
   // tolerance of 1e-6 for 126 to over 200 iterations.  A loose linear
   // tolerance keeps the product, whose error is second order in the residual.
+  // On ill-conditioned models the true residual is far above the tolerance,
+  // which the recurrence meets (1e-9 to 1e-7); what is left is rounding, which
+  // the lowest modes hardly see: relative errors of the four lowest eigenvalues
+  // of cantilevers of 40 and 80 hex8 elements and a plate of thickness 1/200,
+  // against extended precision, up to 8e-11, 3e-10 and 2e-10, by the product 5e-11,
+  // 6e-10 and 1e-10; 4, 4 and 8 iterations, by the product over 30.
   const bool kp_from_rhs = lin.tol > 0 && lin.tol <= 1e-12;
   {
     cudaError_t e = cudaMalloc((void **)&d_X, vb * q);
