@@ -882,6 +882,7 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
     CK(ensure_soa(*c, FAST_ASM_STIFFNESS, mixed));
   }
   const int chunk = opts.check_every > 0 ? opts.check_every : (mixed ? 50 : 32);
+  c->chunk_asked = opts.check_every > 0;
   fast_gpu_solve_report R{};
   if (mixed) {
     CK(pcg_mixed(*c, warm, tol, maxit, chunk));

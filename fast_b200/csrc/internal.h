@@ -260,6 +260,7 @@ struct Ctx {
   bool mf_fp32 = false;          // the solve at hand iterates in FP32
   bool mf_used = false;          // the last solve did
 
+  bool chunk_asked = false;      // the solve at hand has a caller's own check_every
   int products[2] = {0, 0};      // fast_gpu_mult_vect with the present K, M from their blocks
   int64_t launches = 0;          // kernels launched by this context (all entry points)
 

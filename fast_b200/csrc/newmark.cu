@@ -201,6 +201,7 @@ static int graph_steps(fast_gpu_ctx *c, const fast_gpu_newmark_opts *o, int firs
   // 16 below 1e-10, where the FP32 iteration needs the more frequent
   // corrections (the damped box to 1e-12 stops converging with 50)
   const int chunk = lo.check_every > 0 ? lo.check_every : (mixed ? (tol < 1e-10 ? 16 : 50) : 32);
+  c->chunk_asked = lo.check_every > 0;
   const int64_t before = c->launches;
   int64_t per_step = 0;
   NMCK(cudaMalloc((void **)&d_stats, sizeof(h_stats)));

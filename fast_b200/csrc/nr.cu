@@ -147,6 +147,7 @@ static cudaError_t capture_iteration(Ctx &c, NrWork &w, const fast_gpu_nr_opts *
   // the PCG iterations), every 16 for linear tolerances below 1e-10, which
   // need the more frequent corrections
   const int chunk = lo.check_every > 0 ? lo.check_every : (mixed ? (lo.tol > 0 && lo.tol < 1e-10 ? 16 : 50) : 32);
+  c.chunk_asked = lo.check_every > 0;
   const double tol = o->tol > 0 ? o->tol : 1e-5;
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal);

@@ -2187,6 +2187,12 @@ static void mixed_chunk(Ctx &c, int k) {
   mixed_reliable(c);
 }
 
+// FP64 iterations in one launch of the persistent kernel.  A launch ends by
+// itself when the solve does, and each one copies the matrix to shared memory
+// anew: 512 iterations instead of 64 take 3.53 -> 3.36 ms for 624 (hex8 20x4x4),
+// 4.49 -> 4.32 for 575 (hex20 13x9x7).  A caller's own period is kept to, from 64.
+static int persist_chunk(const Ctx &c, int chunk) { return std::max(chunk, c.chunk_asked ? 64 : 512); }
+
 cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int iter0) {
   cudaError_t e;
   fp64_init(c, warm, tol, nullptr, maxit, iter0);
@@ -2197,11 +2203,7 @@ cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int it
       return cudaGetLastError();
     });
   if (use_persistent(c)) {
-    // a launch ends by itself when the solve does, and each one copies the matrix
-    // to shared memory anew: 512 iterations instead of 64 take 3.53 -> 3.36 ms for
-    // 624 (hex8 20x4x4), 4.49 -> 4.32 for 575 (hex20 13x9x7)
-    const int pchunk = std::max(chunk, 512);
-    return drive(c, maxit, pchunk, nullptr, nullptr, nullptr, [&](int k) -> cudaError_t {
+    return drive(c, maxit, persist_chunk(c, chunk), nullptr, nullptr, nullptr, [&](int k) -> cudaError_t {
       return launch_persistent<double>(c, c.d_Ks, c.d_u, c.d_r, c.d_z, c.d_p, c.d_p2, c.d_w, c.d_dinv, k);
     });
   }
@@ -2287,7 +2289,7 @@ cudaError_t record_pcg(Ctx &c, bool mixed, bool warm, double tol, const double *
       mixed_reliable(c);
     } else if (persist) {
       el = launch_persistent<double>(c, c.d_Ks, c.d_u, c.d_r, c.d_z, c.d_p, c.d_p2, c.d_w, c.d_dinv,
-                                     std::max(chunk, 512));
+                                     persist_chunk(c, chunk));
     } else if (mixed) {
       mixed_chunk(c, chunk);
     } else {

@@ -166,7 +166,10 @@ typedef struct {
   double  inner_tol;      /* reserved, 0                                          */
   int32_t max_outer;      /* reserved, 0                                          */
   int32_t check_every;    /* iterations per chunk: convergence read-back period and,
-                             mixed, FP64 residual replacement period; 0 = 32 (FP64) / 50 (mixed) */
+                             mixed, FP64 residual replacement period; 0 = 32 (FP64) / 50 (mixed).
+                             In FP64, systems of at most FAST_OPT_PERSISTENT_MAX_NODES nodes iterate
+                             in one kernel, which stops by itself: 512 iterations a launch (0), or
+                             this many, at least 64 */
 } fast_gpu_solve_opts;
 
 typedef struct {
