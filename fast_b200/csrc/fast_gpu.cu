@@ -888,21 +888,26 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
     CK(pcg_mixed(*c, warm, tol, maxit, chunk));
     R.outer = c->h_state->updates;
     int done = c->h_state->done, it = c->h_state->iter;
+    // the FP64 stiffness in the tensor-core one's place, with its preconditioner
+    auto assemble_fp64 = [&]() -> cudaError_t {
+      cudaError_t e = c->use_first_touch() ? cudaSuccess : launch_zero_matrix(*c, c->d_K, true);
+      if (e == cudaSuccess) e = launch_assemble(*c, FAST_ASM_STIFFNESS, c->d_K);
+      if (e != cudaSuccess) return e;
+      c->K_ok = true;
+      c->K32_current = false;
+      invalidate(*c, FAST_ASM_STIFFNESS);
+      c->K_pure = true;
+      R.escalated |= 2;
+      return launch_build_precond(*c, c->d_K, precond);
+    };
     if ((done == 3 || done == 4) && it < maxit && k32 && !mf) {
       // The tensor-core FP32 stiffness (entries to about 1e-6 of the largest
       // on degree-3 B-splines) could not take this system to the tolerance
       // against its element-by-element FP64 residual, restarts included:
       // assemble the FP64 stiffness and go on with the mixed iteration on it
       // from the best FP64 iterate seen (its FP32 copy is the rounded FP64 K).
-      R.escalated = 2;
       CK(cudaMemcpyAsync(c->d_u, c->d_ubest, sizeof(double) * 4 * c->nnode, cudaMemcpyDeviceToDevice, c->stream));
-      if (!c->use_first_touch()) CK(launch_zero_matrix(*c, c->d_K, true));
-      CK(launch_assemble(*c, FAST_ASM_STIFFNESS, c->d_K));
-      c->K_ok = true;
-      c->K32_current = false;
-      invalidate(*c, FAST_ASM_STIFFNESS);
-      CK(launch_build_precond(*c, c->d_K, precond));
-      c->precond_built = precond;
+      CK(assemble_fp64());
       CK(ensure_soa(*c, FAST_ASM_STIFFNESS, true));
       CK(pcg_mixed(*c, true, tol, maxit - it, chunk));
       R.outer += c->h_state->updates;
@@ -915,6 +920,11 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
       // with the FP64 iteration from the best FP64 iterate seen
       R.escalated |= 1;
       CK(cudaMemcpyAsync(c->d_u, c->d_ubest, sizeof(double) * 4 * c->nnode, cudaMemcpyDeviceToDevice, c->stream));
+      if (mf && c->K32_current) {
+        // (the operator needs no matrix, but a caller finds the stiffness that an escalated solve leaves)
+        CK(assemble_fp64());
+        CK(mf_prepare(*c, mixed, precond));
+      }
       CK(pcg_fp64(*c, true, tol, maxit, chunk, it));
     }
   } else {

@@ -36,7 +36,33 @@ def test_no_restarts_on_the_matrix_free_operator():
     s.upload(d)
     s.assemble(gpu.ASM_K_TF32)
     u, rep = s.solve(f, tol=1e-8, precision=gpu.PREC_MIXED)
-    assert rep["converged"] and rep["escalated"] == 1 and rep["outer"] < 400
+    assert rep["converged"] and rep["escalated"] & 1 and rep["outer"] < 400
+    s.close()
+
+
+@pytest.mark.parametrize("least", [0, 10 ** 12])
+def test_escalated_solve_leaves_the_fp64_stiffness(least):
+    """A mixed solve on the tensor-core stiffness that FP32 cannot finish
+    assembles the FP64 one, matrix-free or not: FP64 solves and products are
+    refused before it and taken after it."""
+    d, f = _model("hex20", (60, 3, 3), (60.0, 3.0, 3.0))
+    s = gpu.GpuSystem(0)
+    s.set_option(gpu.OPT_MATRIX_FREE, least)
+    s.upload(d)
+    s.assemble(gpu.ASM_K_TF32)
+    for call in (lambda: s.solve(f, tol=1e-8), lambda: s.mult_vect(f)):
+        with pytest.raises(gpu.FastGpuError) as e:
+            call()
+        assert e.value.rc == -4
+    u, rep = s.solve(f, tol=1e-10, precision=gpu.PREC_MIXED)
+    assert rep["converged"] and rep["escalated"] & 2
+    v, rep = s.solve(f, tol=1e-10)
+    assert rep["converged"]
+    y = s.mult_vect(f)
+    s.assemble()
+    assert np.array_equal(s.mult_vect(f), y)
+    w, _ = s.solve(f, tol=1e-10)
+    assert np.array_equal(v, w)
     s.close()
 
 
