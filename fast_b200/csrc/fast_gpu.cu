@@ -861,20 +861,23 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
     CK(k32 ? launch_build_precond32(*c, c->d_K32, precond) : launch_build_precond(*c, c->d_K, precond));
   c->mf_fp32 = mixed;
   bool mf = mf_active(*c);
-  // without memory for its operands this solve goes to the assembled matrix, whose layout may be there
-  const OnAssembledMatrix restore(*c);
-  c->mf_off = restore.was;
   if (mf) {
     const cudaError_t e = mf_prepare(*c, mixed, precond);
+    // without memory for its operands this solve goes to the assembled matrix, whose layout may be there
     if (e == cudaErrorMemoryAllocation) {
       mf_give_up(*c);
       mf = false;
-      c->mf_off = true;
     } else {
       CK(e);
     }
   }
   c->mf_used = mf;
+  // decided once, behind the set-up: nothing the solve does to the matrix turns it on without
+  struct Scope {
+    Ctx &c;
+    ~Scope() { c.mf_on = false; }
+  } scope{*c};
+  c->mf_on = mf;
   if (mf) {
     if (c->graph_mf_precond != precond) c->drop_graphs();
     c->graph_mf_precond = precond;
@@ -896,7 +899,7 @@ int solve_node_space(fast_gpu_ctx *c, const fast_gpu_solve_opts *o, bool warm, f
       c->K_ok = true;
       c->K32_current = false;
       invalidate(*c, FAST_ASM_STIFFNESS);
-      c->K_pure = true;
+      c->K_pure = true;  // (the next solve may be matrix-free)
       R.escalated |= 2;
       return launch_build_precond(*c, c->d_K, precond);
     };

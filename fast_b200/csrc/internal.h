@@ -258,7 +258,8 @@ struct Ctx {
   bool mf_off = false;           // a driver that edits or replays the matrix itself is running
   int64_t mf_min_nodes = -1;     // systems this large take it (-1: the measured default)
   bool mf_fp32 = false;          // the solve at hand iterates in FP32
-  bool mf_used = false;          // the last solve did
+  bool mf_on = false;            // the solve at hand is matrix-free (its operands are prepared)
+  bool mf_used = false;          // the last solve was
 
   bool chunk_asked = false;      // the solve at hand has a caller's own check_every
   int products[2] = {0, 0};      // fast_gpu_mult_vect with the present K, M from their blocks
@@ -486,8 +487,8 @@ cudaError_t launch_matfree_residual(Ctx &c, const double *f, const double *u, do
                                     const int32_t *skip);
 // AoS blocks -> row-local SoA copies (either output may be null)
 cudaError_t launch_to_soa(Ctx &c, const double *K, double *Ks, float *Ks32);
-// matfree.cu: whether the solve of the current stiffness runs matrix-free; its
-// operands (also the preconditioner's compact diagonal); k iterations from the
+// matfree.cu: whether a solve of the current stiffness runs matrix-free (the
+// solve at hand: Ctx::mf_on); its operands (also the preconditioner's compact diagonal); k iterations from the
 // direction p (pcg_direction_fused has to follow: the last update's sums are in
 // part_rr and part_zr); r = f - K u with r.r in nparts partials, nothing while
 // *skip

@@ -1076,7 +1076,7 @@ cudaError_t launch_spmv32(Ctx &c, const float *Ks, const float *x, float *y) {
 
 cudaError_t launch_residual(Ctx &c, const double *Ks, const double *f, const double *u, double *r, double *rr_out) {
   double *part = P_E(c);
-  if (mf_active(c)) {
+  if (c.mf_on) {
     cudaError_t e = mf_residual_of(c, f, u, r, part, spmv_grid(c), nullptr);
     if (e != cudaSuccess) return e;
   } else if (Ks) {
@@ -2075,7 +2075,7 @@ static void fp64_init(Ctx &c, bool warm, double tol, const double *tol_dev, int 
   const int64_t nn = c.nnode;
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
-  if (warm && mf_active(c)) {
+  if (warm && c.mf_on) {
     mf_residual_of(c, c.d_f, c.d_u, c.d_r, P_E(c), G, nullptr);
   } else if (warm) {
     spmv64_go<1>(c, G, nn, c.d_Ks, c.d_u, c.d_f, c.d_r, P_E(c), nullptr);
@@ -2094,7 +2094,7 @@ static void fp64_chunk(Ctx &c, int k) {
   const int64_t nn = c.nnode;
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
-  if (mf_active(c)) {
+  if (c.mf_on) {
     mf_iterations<double>(c, k, c.d_u, c.d_r, c.d_z, c.d_p, P_A(c), P_B(c), P_C(c));
     pcg_direction_fused<double><<<R, kVecThreads, 0, c.stream>>>(nn, c.d_p, c.d_z, st, P_B(c), P_C(c), R);
     c.launches++;
@@ -2132,7 +2132,7 @@ static void mixed_init(Ctx &c, bool warm, double tol, const double *tol_dev, int
   // the tensor-core stiffness may restart its recurrence (see reliable_scalar);
   // the matrix-free operator is the same in both precisions
   mixed_init_scalar<<<1, 256, 0, c.stream>>>(c.d_state, P_D(c), R, tol, tol_dev, maxit,
-                                             c.K32_current && !mf_active(c) ? 40 : 0, plateau);
+                                             c.K32_current && !c.mf_on ? 40 : 0, plateau);
   c.launches += 2;
 }
 
@@ -2144,7 +2144,7 @@ static void mixed_reliable(Ctx &c) {
   const int G = spmv_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
   flush_correction<<<R, 256, 0, c.stream>>>(4 * nn, c.d_u, c.s_x, st);
-  if (mf_active(c)) {
+  if (c.mf_on) {
     mf_residual_of(c, c.d_f, c.d_u, c.d_r, P_E(c), G, &st->final);
   } else if (c.K32_current) {
     launch_matfree_residual(c, c.d_f, c.d_u, c.d_r, P_E(c), &st->final);  // counts its own launches
@@ -2168,7 +2168,7 @@ static void mixed_chunk(Ctx &c, int k) {
   const int64_t nn = c.nnode;
   const int G = spmv32_grid(c), R = kRedBlocks;
   PcgState *st = c.d_state;
-  if (mf_active(c)) {
+  if (c.mf_on) {
     mf_iterations<float>(c, k, c.s_x, c.s_r, c.s_z, c.s_p, P_A(c), P_B(c), P_C(c));
     pcg_direction_fused<float><<<R, kVecThreads, 0, c.stream>>>(nn, c.s_p, c.s_z, st, P_B(c), P_C(c), R);
     c.launches++;
@@ -2197,7 +2197,7 @@ cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int it
   cudaError_t e;
   fp64_init(c, warm, tol, nullptr, maxit, iter0);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (mf_active(c))
+  if (c.mf_on)
     return drive(c, maxit, chunk, &c.graph_mf64, &c.graph_mf64_chunk, &c.graph_mf64_kernels, [&](int k) -> cudaError_t {
       fp64_chunk(c, k);
       return cudaGetLastError();
@@ -2216,10 +2216,10 @@ cudaError_t pcg_fp64(Ctx &c, bool warm, double tol, int maxit, int chunk, int it
 // FP32 PCG with FP64 reliable updates every `chunk` iterations.
 cudaError_t pcg_mixed(Ctx &c, bool warm, double tol, int maxit, int chunk) {
   cudaError_t e;
-  mixed_init(c, warm, tol, nullptr, maxit, !mf_active(c) && use_persistent(c) ? kPlateauPersistent : kPlateau);
+  mixed_init(c, warm, tol, nullptr, maxit, !c.mf_on && use_persistent(c) ? kPlateauPersistent : kPlateau);
   mixed_reliable(c);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (mf_active(c))
+  if (c.mf_on)
     return drive(c, maxit, chunk, &c.graph_mf32, &c.graph_mf32_chunk, &c.graph_mf32_kernels, [&](int k) -> cudaError_t {
       mixed_chunk(c, k);
       return cudaGetLastError();
@@ -2256,7 +2256,7 @@ cudaError_t record_pcg(Ctx &c, bool mixed, bool warm, double tol, const double *
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // small systems iterate in the persistent cooperative kernel (as the
   // launched solves do), a chunk per loop pass
-  const bool persist = !mf_active(c) && use_persistent(c);
+  const bool persist = !c.mf_on && use_persistent(c);
   // the WHILE node, appended to the graph being captured on c.stream
   cudaStreamCaptureStatus cs;
   cudaGraph_t g = nullptr;

@@ -66,6 +66,29 @@ def test_escalated_solve_leaves_the_fp64_stiffness(least):
     s.close()
 
 
+def test_matrix_free_is_decided_once():
+    """A solve that began on an assembled matrix stays on it, also where it
+    assembles the FP64 stiffness on the way: here on the tensor-core matrix, after
+    a transient analysis that was refused has changed the FP64 slot."""
+    d, f = _model("hex20", (60, 3, 3), (60.0, 3.0, 3.0))
+    d.rho = np.full(len(d.conn), 1e-3)
+    s = gpu.GpuSystem(0)
+    s.set_option(gpu.OPT_MATRIX_FREE, 0)
+    s.upload(d)
+    s.assemble(gpu.ASM_K_TF32)
+    with pytest.raises(gpu.FastGpuError) as e:
+        s.newmark(f, 2, 1e-3)
+    assert e.value.rc == -4
+    before = s.launch_count()
+    u, rep = s.solve(f, tol=1e-10, precision=gpu.PREC_MIXED)
+    assert rep["converged"] and rep["escalated"] & 2
+    # the persistent kernel: far fewer launches than the two an iteration of a matrix-free solve
+    assert s.launch_count() - before < rep["iterations"]
+    v, rep = s.solve(f, tol=1e-10, precision=gpu.PREC_MIXED)
+    assert rep["converged"] and np.linalg.norm(u - v) <= 1e-6 * np.linalg.norm(v)
+    s.close()
+
+
 @pytest.mark.parametrize("kind,n,L", [("hex8", (200, 2, 2), (200.0, 2.0, 2.0)), ("hex20", (60, 3, 3), (60.0, 3.0, 3.0)),
                                       ("hex8", (60, 60, 1), (60.0, 60.0, 0.5))])
 def test_persistent_kernel_gives_up_after_ten(kind, n, L):
