@@ -812,7 +812,7 @@ int fast_gpu_get(fast_gpu_ctx *c, int32_t what, int32_t i, int32_t j, double *v)
 int fast_gpu_mult_vect(fast_gpu_ctx *c, int32_t what, const double *x, double *y) {
   if (check_ctx(c) || !x || !y) return FAST_GPU_EINVAL;
   double *T = target_of(*c, what);
-  if (!T || (what == FAST_ASM_STIFFNESS && !c->K_ok) || (what == FAST_ASM_MASS && !c->M_ok)) return FAST_GPU_ESTATE;
+  if (!T || (what == FAST_ASM_STIFFNESS && (!c->K_ok || c->K32_current)) || (what == FAST_ASM_MASS && !c->M_ok)) return FAST_GPU_ESTATE;
   const size_t nb = sizeof(double) * c->neq;
   CK(cudaStreamSynchronize(c->stream));
   copy_host(c->h_eq_tmp, x, nb);

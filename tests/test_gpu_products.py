@@ -58,3 +58,18 @@ def test_products_have_the_same_bits(name, lanes):
     # rows of at most 343 blocks in FP64
     assert np.all(np.abs(full @ x - first[gpu.ASM_K]) <= 3 * 343 * 2.0 ** -52 * (abs(full) @ np.abs(x)))
     s.close()
+
+
+def test_no_product_with_an_edited_slot_behind_the_tensor_core_stiffness():
+    """While the tensor-core stiffness is the context's, the FP64 slot is not:
+    no product with it, also when a refused transient analysis has filled it."""
+    d = _box("hex20", (4, 3, 2))
+    x = np.ones(d.num_eq())
+    s = gpu.GpuSystem(0)
+    s.upload(d)
+    s.assemble(gpu.ASM_K_TF32)
+    for call in (lambda: s.mult_vect(x), lambda: s.newmark(x, 2, 1e-3), lambda: s.mult_vect(x)):
+        with pytest.raises(gpu.FastGpuError) as e:
+            call()
+        assert e.value.rc == -4
+    s.close()
