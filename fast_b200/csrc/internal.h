@@ -320,7 +320,7 @@ struct Ctx {
   uint16_t *d_lcol = nullptr;     // [nnzb_pad] its list indices of the matrix columns
   double *d_z2 = nullptr;         // [nnode][4] its second z buffer (either precision)
   void *d_bar = nullptr;          // exchange words of that kernel (kBarrierBytes)
-  static constexpr size_t kBarrierBytes = 16384;
+  static constexpr size_t kBarrierBytes = 128;
 
   // CUDA graphs of one chunk of PCG iterations (captured once, replayed)
   cudaGraphExec_t graph_fp64 = nullptr, graph_mixed = nullptr;

@@ -6,8 +6,9 @@
 // 131,072 elements, 214 / 402 us at 6 TB/s.  Applied element by element
 // (matfree_math.cuh) the same product reads 9 numbers per Gauss point and the
 // directions of the element's nodes: 0.19 / 0.37 GB, and about 4,700
-// multiply-adds per element.  Measured there: element kernel 66 / 110 us, node
-// kernel 27 / 52 us (an iteration 239 -> 98 us in FP32, 447 -> 168 us in FP64).
+// multiply-adds per element.  Measured there: element kernel 68 / 117 us, node
+// kernel 27 / 51 us (an iteration 239 -> 102 us in FP32, with its FP64 residuals,
+// 447 -> 173 us in FP64).
 // What bounds the element kernel now is the latency of its dependent steps at
 // 12 (9) warps per SM: with the geometry resident in L2 it still takes 62 us.
 //

@@ -1168,9 +1168,9 @@ cudaError_t launch_build_precond32(Ctx &c, const float *K32, int precond) {
 // those of pcg_update_fused / pcg_direction_fused; block 0 writes them back to
 // the PcgState at the end.  Measured per iteration (rows split evenly, matrix
 // and gathers through L2, release counters and partials read back -> this):
-// hex8 plate tangent, 7,605 nodes, FP32 10.0 -> 6.4 us; hex20, 40,623 nodes,
-// FP32 33.5 -> 19; tied column, 12,526 nodes, FP32 32.6 -> 13; hex20, 4,148
-// nodes, FP64 14.8 -> 7.1; hex8, 525 nodes, FP64 8.8 -> 5.0.
+// hex8 plate tangent, 7,605 nodes, FP32 10.0 -> 5.7 us; hex20, 40,623 nodes,
+// FP32 33.5 -> 17.8, and 30,600 nodes 23 -> 14.4; tied column, 12,526 nodes, FP32
+// 32.6 -> 9.9; hex20, 4,148 nodes, FP64 14.8 -> 7.0; hex8, 525 nodes, FP64 8.8 -> 5.0.
 constexpr int kPersistThreads = 512;
 constexpr int kPersistSmem = 208 * 1024;   // dynamic shared memory of a block
 constexpr int kPersistRows = 1024;         // resident rows at most (their offsets are kept)
@@ -1181,9 +1181,8 @@ template <typename T> constexpr int kHaloMax = sizeof(T) == 4 ? 4096 : 2560;  //
 constexpr long long kWaitCycles = 4000000000ll;  // about 2 s of SM clock in one wait; then the launch gives up
 
 // Words of grid_sum: [2 sets][2 values][3 limbs], zeroed before a launch.
-constexpr int kSumStride = 1;
 struct GridSlots {
-  unsigned long long w[2 * 6 * kSumStride];
+  unsigned long long w[2 * 6];
 };
 static_assert(sizeof(GridSlots) <= Ctx::kBarrierBytes, "grid_sum words exceed their allocation");
 constexpr int kMaxCluster = 16, kMaxSumBlocks = 148;
@@ -1231,8 +1230,8 @@ __device__ __forceinline__ void cluster_barrier() {
 // still waits for.  Measured on 148 blocks (cycles): release counter and
 // polls 2,790, then the partials read back 760; these words 1,700 (2,550
 // ORDERED); flags posted by every block and polled by every block 5,000 to
-// 12,000.  Every wait is bounded: when one runs out the block leaves, and the
-// others, whose waits then run out too, follow.
+// 12,000.  Every wait is bounded, by SM cycles: when one runs out the block
+// leaves without a word to the others, whose own waits run out in turn.
 //
 // A grid of one cluster exchanges its partials through distributed shared
 // memory between two hardware barriers instead.
@@ -1290,7 +1289,7 @@ __device__ bool grid_sum(GridSlots *S, SumShared &sh, int CS, int rank, SumState
       st.phase++;
       const double x = (NV > 1 && k0) ? t[NV - 1] : t[0];
       const int e = (NV > 1 && k0) ? E[NV - 1].e : E[0].e;
-      unsigned long long *w = &S->w[(par * 6 + (mine ? lane : 0)) * kSumStride];
+      unsigned long long *w = &S->w[par * 6 + (mine ? lane : 0)];
       const long long add = sum_limb(x, e, limb);
       unsigned long long cur = 0;
       const unsigned long long seen = par ? st.seen[1] : st.seen[0];

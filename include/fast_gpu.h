@@ -18,6 +18,11 @@
  *   - Matrix indices (i, j) are 0-based equation indices, as in
  *     cSysMatrix::Add/Get (mlib/sysmat.h:85-86).
  *   - The context owns all device memory; one context serves one host thread.
+ *   - Copies of 3 MB and more between a caller's arrays and the pinned staging
+ *     buffer are shared by up to eight OpenMP threads of the calling process
+ *     (OMP_NUM_THREADS limits them), in every call that takes or returns vectors.
+ *   - A change of stream (fast_gpu_set_stream) waits for copies still on their
+ *     way from that buffer; work already launched is the caller's to order.
  *   - Calls are stream-ordered on the context's stream; calls that return
  *     host data synchronise that stream.  Every device wait is bounded.
  */
@@ -224,7 +229,15 @@ int         fast_gpu_synchronize(fast_gpu_ctx *ctx);
                                             without ties, on the stiffness as last assembled: from this many
                                             nodes on K.u is applied element by element instead of by the
                                             assembled matrix (the same operator to rounding); -1 (default):
-                                            from where it was measured faster */
+                                            from where it was measured faster.  Steers fast_gpu_solve,
+                                            fast_gpu_solve_device, the linear solves of fast_gpu_modal and
+                                            fast_gpu_buckling and, for hex8, fast_gpu_solve_batch (nodes of
+                                            all problems).  A mixed solve then rounds the geometry of each
+                                            Gauss point and the element forces to FP32 instead of the
+                                            blocks of K (its FP64 residuals are FP64 as before); after
+                                            FAST_ASM_STIFFNESS_TF32 it takes only the preconditioner from the
+                                            tensor-core matrix.  Without memory for its operands a solve
+                                            goes to the assembled matrix */
 #define FAST_OPT_PERSISTENT_ASSEMBLY  8  /* 1: FAST_ASM_STIFFNESS_TF32 integrates the elements of every
                                             bucket in one persistent cooperative launch (colour k of
                                             every bucket is phase k, grid barriers between phases, CTAs
@@ -595,7 +608,9 @@ int fast_gpu_add(fast_gpu_ctx *ctx, int32_t what, int32_t i, int32_t j, double v
 int fast_gpu_add_mat(fast_gpu_ctx *ctx, int32_t dst, double a, int32_t src);
 /* cSysMatrix::Get(i, j) */
 int fast_gpu_get(fast_gpu_ctx *ctx, int32_t what, int32_t i, int32_t j, double *v);
-/* cSysMatrix::MultVect(in, out): out = K in, equation space, host buffers. */
+/* cSysMatrix::MultVect(in, out): out = K in, equation space, host buffers.
+ * The bits do not depend on the solves before it; after 12 products with the
+ * same matrix its solve layout is made (76 bytes a block), if it finds memory. */
 int fast_gpu_mult_vect(fast_gpu_ctx *ctx, int32_t what, const double *x, double *y);
 /* cSysMatrix::Solve(b, x) (mlib/sysmat.cpp:966-970 -> PCGSolver :1061-1125):
  * host f and u of length num_eq. */
