@@ -93,9 +93,9 @@ FG_HD bool sum_again(SumScale &s, bool over, double &res) {
     s.e = s.e + 64 < s.fit ? s.e + 64 : s.fit;
     return true;
   }
-  s.fit = s.e;
   const int re = double_exponent(res);
-  if (s.up || re >= s.e - 66 || s.e <= kScaleMin) return false;
+  if (re >= s.e - 66 || s.up || s.e <= kScaleMin) return false;
+  s.fit = s.e;
   const int e = res != 0.0 ? re + 20 : s.e - 60;
   s.e = e > kScaleMin ? e : kScaleMin;
   return true;
